@@ -506,8 +506,8 @@ def run_ours(args, world, rank, local):
 
     if rank != 0:
         return
-    # roofline of the dominant stage (the peel: k_peel and, when it stops
-    # early, the endgame kernels that finish the columns): algorithmic bytes
+    # roofline of the dominant stage (the peel: k_peel and the late form that
+    # finishes the columns, or takes every level): algorithmic bytes
     # per launch (bytes_per_column per lambda column) over the mean CUDA-event
     # time of a launch
     cols = min(stats["columns_per_launch"] or L, max(my_cols, 1))
@@ -519,8 +519,8 @@ def run_ours(args, world, rank, local):
                              else (None, None))
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak, "traffic": traffic,
-            "kernel": "k_peel + endgame (k_eg_index, k_eg_scan, k_eg_fill, k_eg_fill_big, "
-                      "k_endgame)", "peak_kind": peak_kind,
+            "kernel": "k_peel + late form (k_lt_rows, k_lt_degrees, k_lt_fill, k_lt_fill_long, "
+                      "k_late)", "peak_kind": peak_kind,
             "bytes_per_launch": bytes_per_launch, "launch_ms": launch_ms,
             # atomics are reported beside the bytes, not folded in
             "l2_atomic_sectors_per_launch": atom_sectors,
@@ -749,7 +749,7 @@ def run_batch(args, world, rank, local):
             "plain_per_graph": {"ms": plain_graph_ms,
                                 "form": "one graph per call of the single-graph path "
                                         "(fc_coreindex: all its columns in one launch with the "
-                                        "endgame, then fc_densest), graph after graph"},
+                                        "late form, then fc_densest), graph after graph"},
             "plain_per_column": {"ms": plain_col_ms, "report": plain_rep,
                                  "form": "one graph and one lambda column per launch"},
             "speedup_vs_plain_per_graph": (plain_graph_ms / ms) if plain_graph_ms else None,

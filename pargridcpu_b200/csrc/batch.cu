@@ -150,7 +150,7 @@ static fc_status batch_plain(fc_graph* const* gs, uint32_t count, double beta,
     double peel_ms = 0;
     uint32_t launches = 0, levels = 0;
     for (uint32_t i = 0; i < count; i++)
-        FC_TRY(batch_plain_one(gs[i], s, &peel_ms, &launches, &levels));
+        FC_TRY(batch_plain_one(gs[i], s, &peel_ms, &launches, &levels, true));
     double dms = 0;
     const auto t_dense = std::chrono::steady_clock::now();
     FC_TRY(densest_all(gs, count, beta, res, s, &dms));
@@ -181,15 +181,16 @@ static std::mutex g_tune_mu;
 static std::map<TuneKey, std::pair<uint32_t, uint32_t>> g_tuned;  // -> (threads, small_row)
 
 // Launch groups: consecutive graphs whose peel scratch stays within the
-// budget (FC_BATCH_WS_MB, default 32 GiB) share one launch.
-static void plan_groups(const std::vector<PeelSegSpec>& specs, uint64_t budget,
+// budget (FC_BATCH_WS_MB, default 32 GiB) share one launch, unless one's
+// columns are packed and the other's are not.
+static void plan_groups(const std::vector<PeelSegSpec>& specs, uint64_t budget, bool late,
                         std::vector<std::pair<size_t, size_t>>* groups) {
     size_t i = 0;
     while (i < specs.size()) {
         size_t e = i + 1;
-        while (e < specs.size()) {
+        while (e < specs.size() && peel_packs(specs[e], late) == peel_packs(specs[i], late)) {
             std::vector<PeelSegSpec> trial(specs.begin() + i, specs.begin() + e + 1);
-            if (peel_batch_ws_bytes(trial) > budget) break;
+            if (peel_batch_ws_bytes(trial, late) > budget) break;
             e++;
         }
         groups->push_back({i, e});
@@ -200,7 +201,7 @@ static void plan_groups(const std::vector<PeelSegSpec>& specs, uint64_t budget,
 static fc_status run_groups(const std::vector<PeelSegSpec>& specs,
                             const std::vector<std::pair<size_t, size_t>>& groups, void* ws,
                             uint64_t ws_bytes, cudaStream_t s, uint32_t threads, uint32_t small_row,
-                            bool want_graph, uint32_t max_sms, double* ms, uint32_t* levels,
+                            bool want_graph, uint32_t max_sms, bool late, double* ms, uint32_t* levels,
                             bool* graphed) {
     *ms = 0;
     *levels = 0;
@@ -211,7 +212,7 @@ static fc_status run_groups(const std::vector<PeelSegSpec>& specs,
         bool g = want_graph;
         BATCH_TRACE("peel graphs [%zu, %zu) threads %u small_row %u graph %d", gr.first,
                     gr.second, threads, small_row, (int)g);
-        FC_TRY(peel_batch(part, ws, ws_bytes, s, &st, threads, small_row, &g, max_sms));
+        FC_TRY(peel_batch(part, ws, ws_bytes, s, &st, threads, small_row, &g, max_sms, late));
         BATCH_TRACE("  done: %.3f ms, %u levels, cuda graph %d", st.ms, st.levels, (int)g);
         *graphed = *graphed && g;
         *ms += st.ms;
@@ -220,7 +221,7 @@ static fc_status run_groups(const std::vector<PeelSegSpec>& specs,
     return FC_OK;
 }
 
-uint64_t batch_peel_ws_bytes(fc_graph* const* gs, uint32_t count) {
+uint64_t batch_peel_ws_bytes(fc_graph* const* gs, uint32_t count, bool late) {
     std::vector<PeelSegSpec> specs;
     for (uint32_t i = 0; i < count; i++) {
         const fc_graph* g = gs[i];
@@ -229,14 +230,24 @@ uint64_t batch_peel_ws_bytes(fc_graph* const* gs, uint32_t count) {
         sp.g.n = g->n;
         sp.g.L = g->L;
         sp.g.entries = g->total_entries();
+        sp.g.max_level = g->n;  // the degrees are only known on the device
         sp.ncols = g->L;
         specs.push_back(sp);
     }
-    return specs.empty() ? 0 : peel_batch_ws_bytes(specs);
+    return specs.empty() ? 0 : peel_batch_ws_bytes(specs, late);
+}
+
+uint64_t plain_peel_ws_bytes(const fc_graph* g, bool late) {
+    PeelGraph p{};
+    p.n = g->n;
+    p.L = g->L;
+    p.entries = g->total_entries();
+    p.max_level = g->n;
+    return peel_ws_bytes(p, 1, late);
 }
 
 fc_status batch_peel(fc_graph* const* gs, uint32_t count, const fc_batch_options* opt,
-                     uint32_t max_sms, fc_batch_report* rep, cudaStream_t s) {
+                     uint32_t max_sms, fc_batch_report* rep, cudaStream_t s, bool late) {
     std::vector<PeelSegSpec> specs;
     uint32_t maxL = 1;
     uint64_t entries = 0;
@@ -260,16 +271,25 @@ fc_status batch_peel(fc_graph* const* gs, uint32_t count, const fc_batch_options
     }
     const uint64_t budget = (uint64_t)env_u32b("FC_BATCH_WS_MB", 32768) << 20;
     std::vector<std::pair<size_t, size_t>> groups;
-    plan_groups(specs, budget, &groups);
     uint64_t ws_bytes = 0;
-    for (const auto& gr : groups) {
-        std::vector<PeelSegSpec> part(specs.begin() + gr.first, specs.begin() + gr.second);
-        ws_bytes = std::max(ws_bytes, peel_batch_ws_bytes(part));
+    void* ws = nullptr;
+    for (;;) {  // without the late form's scratch when there is no room for it
+        groups.clear();
+        ws_bytes = 0;
+        plan_groups(specs, budget, late, &groups);
+        for (const auto& gr : groups) {
+            std::vector<PeelSegSpec> part(specs.begin() + gr.first, specs.begin() + gr.second);
+            ws_bytes = std::max(ws_bytes, peel_batch_ws_bytes(part, late));
+        }
+        if (specs.empty()) break;
+        const fc_status arc = dev_alloc(&ws, ws_bytes, s);
+        if (arc == FC_OK) break;
+        if (arc != FC_ERR_OOM || !late) return arc;
+        cudaGetLastError();
+        late = false;
     }
     BATCH_TRACE("%u graphs uploaded, %zu segments, %zu launch groups, workspace %llu bytes", count,
                 specs.size(), groups.size(), (unsigned long long)ws_bytes);
-    void* ws = nullptr;
-    if (!specs.empty()) FC_TRY(dev_alloc(&ws, ws_bytes, s));
     const bool want_graph = opt ? opt->use_cuda_graph != 0 : true;
     uint32_t threads = opt ? opt->block_threads : 0;
     uint32_t small_row = opt ? opt->hub_threshold : 0;
@@ -289,14 +309,14 @@ fc_status batch_peel(fc_graph* const* gs, uint32_t count, const fc_batch_options
             const size_t step = std::max<size_t>(1, specs.size() / 32);
             for (size_t i = 0; i < specs.size(); i += step) sample.push_back(specs[i]);
             std::vector<std::pair<size_t, size_t>> sg;
-            plan_groups(sample, ws_bytes, &sg);
+            plan_groups(sample, ws_bytes, late, &sg);
             double best_ms = 1e300;
             for (uint32_t th : {512u, 1024u})
                 for (uint32_t sr : {16u, 32u, 64u}) {
                     double ms;
                     uint32_t lv;
                     bool gr;
-                    rc = run_groups(sample, sg, ws, ws_bytes, s, th, sr, false, max_sms, &ms, &lv,
+                    rc = run_groups(sample, sg, ws, ws_bytes, s, th, sr, false, max_sms, late, &ms, &lv,
                                     &gr);
                     if (rc != FC_OK) break;
                     if (ms < best_ms) {
@@ -318,7 +338,7 @@ fc_status batch_peel(fc_graph* const* gs, uint32_t count, const fc_batch_options
     bool graphed = false;
     if (rc == FC_OK && !specs.empty())
         rc = run_groups(specs, groups, ws, ws_bytes, s, threads, small_row, want_graph, max_sms,
-                        &peel_ms, &levels, &graphed);
+                        late, &peel_ms, &levels, &graphed);
     if (ws) dev_free(ws, s);
     FC_TRY(rc);
     for (uint32_t i = 0; i < count; i++) gs[i]->dev->table_valid = true;
@@ -338,7 +358,7 @@ static fc_status batch_persistent(fc_graph* const* gs, uint32_t count, double be
                                   uint32_t* const* tables, fc_densest_result* res,
                                   const fc_batch_options* opt, fc_batch_report* rep,
                                   cudaStream_t s) {
-    FC_TRY(batch_peel(gs, count, opt, 0, rep, s));
+    FC_TRY(batch_peel(gs, count, opt, 0, rep, s, true));
     double dms = 0;
     const auto t_dense = std::chrono::steady_clock::now();
     FC_TRY(densest_all(gs, count, beta, res, s, &dms));
@@ -350,14 +370,14 @@ static fc_status batch_persistent(fc_graph* const* gs, uint32_t count, double be
 }
 
 fc_status batch_plain_one(fc_graph* g, cudaStream_t s, double* peel_ms, uint32_t* launches,
-                          uint32_t* levels) {
+                          uint32_t* levels, bool late) {
     FC_TRY(upload(g, s));
     DeviceGraph* d = g->dev;
     d->home = s;
     invalidate_densest(d);
     for (uint32_t c = 0; c < d->L && d->n; c++) {
         PeelStats st;
-        FC_TRY(peel_columns(d, c, 1, s, &st));
+        FC_TRY(peel_columns(d, c, 1, s, &st, late));
         *peel_ms += st.ms;
         *launches += 1;
         *levels += st.levels;

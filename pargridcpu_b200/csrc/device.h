@@ -152,7 +152,7 @@ struct PeelStats {
     double phase_ms[3] = {0, 0, 0};  // scan, expand, recompute (device timer)
 };
 fc_status peel_columns(DeviceGraph* d, uint32_t col0, uint32_t ncols, cudaStream_t s,
-                       PeelStats* st);
+                       PeelStats* st, bool late = true);
 uint32_t peel_columns_per_group(const DeviceGraph* d);
 
 // A device-resident graph in the kernels' layout, whoever owns the memory.
@@ -167,14 +167,12 @@ struct PeelGraph {
     const uint32_t* big_id = nullptr;
     const uint32_t* ptab = nullptr;
 };
-// scratch bytes one peel launch over `ncols` columns needs
-uint64_t peel_ws_bytes(uint32_t n, uint32_t L, uint64_t entries, uint32_t ncols);
+// scratch bytes one peel launch over `ncols` columns of g needs
+uint64_t peel_ws_bytes(const PeelGraph& g, uint32_t ncols, bool late = false);
 // columns [col0, col0 + ncols) of `table` (lambda-major), scratch in `ws`;
 // allocates nothing unless `instrument` (events; a trace when FC_PEEL_TRACE)
-// or `endgame` (the last levels in one block per column; a temporary buffer
-// when the survivors' subgraphs outgrow the spent queues)
 fc_status peel_run(const PeelGraph& g, uint32_t col0, uint32_t ncols, uint32_t* table, void* ws,
-                   size_t ws_bytes, cudaStream_t s, PeelStats* st, bool instrument, bool endgame);
+                   size_t ws_bytes, cudaStream_t s, PeelStats* st, bool instrument, bool late = false);
 
 // One segment of a batched launch: columns [col0, col0 + ncols) of graph g,
 // written to table (lambda-major, L*n).
@@ -183,7 +181,12 @@ struct PeelSegSpec {
     uint32_t col0, ncols;
     uint32_t* table;
 };
-uint64_t peel_batch_ws_bytes(const std::vector<PeelSegSpec>& specs);
+// `late`: the form that takes a peel's last levels (late.cu) may be used.  Its
+// scratch comes on top of the peel's; without it the peel runs to its end.
+// Whether a launch of such segments packs four columns' degrees in a word
+// (peel.cu); segments that do and segments that do not are not launched together.
+bool peel_packs(const PeelSegSpec& sp, bool late);
+uint64_t peel_batch_ws_bytes(const std::vector<PeelSegSpec>& specs, bool late);
 // All segments in one persistent launch (threads per block and the longest row
 // queued as one item: 0 = defaults).  With *use_graph set the launch is
 // captured in a CUDA graph; on return *use_graph says whether it was.  The grid
@@ -191,7 +194,7 @@ uint64_t peel_batch_ws_bytes(const std::vector<PeelSegSpec>& specs);
 // run beside it.
 fc_status peel_batch(const std::vector<PeelSegSpec>& specs, void* ws, size_t ws_bytes,
                      cudaStream_t s, PeelStats* st, uint32_t threads, uint32_t small_row,
-                     bool* use_graph, uint32_t max_sms = 0);
+                     bool* use_graph, uint32_t max_sms, bool late);
 
 // last CUDA error text, for diagnostics
 const char* last_cuda_error();

@@ -113,13 +113,16 @@ fc_status batch_run(fc_graph* const* gs, uint32_t count, double beta, uint32_t* 
 // at most max_sms SMs (0 = all) on stream s, uploading graphs as needed;
 // each graph's table is valid on the device afterwards.  rep may be NULL.
 fc_status batch_peel(fc_graph* const* gs, uint32_t count, const fc_batch_options* opt,
-                     uint32_t max_sms, fc_batch_report* rep, cudaStream_t s);
+                     uint32_t max_sms, fc_batch_report* rep, cudaStream_t s, bool late);
 // the peel scratch batch_peel allocates for these graphs (one launch group)
-uint64_t batch_peel_ws_bytes(fc_graph* const* gs, uint32_t count);
+// (`late`: with the scratch of the peel's late form, which a run can do without)
+uint64_t batch_peel_ws_bytes(fc_graph* const* gs, uint32_t count, bool late);
+// the scratch of one of g's columns (the plain form)
+uint64_t plain_peel_ws_bytes(const fc_graph* g, bool late);
 // one graph, one lambda column per launch (the plain form); table valid
 // after; adds to the three counters
 fc_status batch_plain_one(fc_graph* g, cudaStream_t s, double* peel_ms, uint32_t* launches,
-                          uint32_t* levels);
+                          uint32_t* levels, bool late);
 // a graph's device copy is going away: servers drop it from their records
 void residency_forget(fc_graph* g);
 // device or pinned-host allocations, streams and events this library created

@@ -91,7 +91,11 @@ extern "C" fc_status fc_coreindex_fixed_scratch(uint32_t n, uint32_t n_layers, u
     // the most columns per launch whose scratch fits the fixed array; a graph
     // whose single column does not fit is rejected before any device work
     uint32_t cols = n_layers;
-    while (cols > 0 && peel_ws_bytes(n, n_layers, entries, cols) > PEEL_SCRATCH_BYTES) cols--;
+    // core <= largest degree <= n - 1 bounds the level count
+    const PeelGraph g{n, n_layers, entries, node_ptr, adj, deg0, n + 1};
+    // (with the form for a peel's last levels when all columns fit with it)
+    const bool late = peel_ws_bytes(g, cols, true) <= PEEL_SCRATCH_BYTES;
+    while (!late && cols > 0 && peel_ws_bytes(g, cols) > PEEL_SCRATCH_BYTES) cols--;
     if (cols == 0) return FC_ERR_TOO_LARGE;
     void* ws = nullptr;
     FC_TRY(fixed_scratch(&ws));
@@ -109,12 +113,10 @@ extern "C" fc_status fc_coreindex_fixed_scratch(uint32_t n, uint32_t n_layers, u
         FC_TRY(to_host(&flag, bad, 4, s));
         if (flag) return FC_ERR_INVALID;
     }
-    // core <= largest degree <= n - 1 bounds the level count
-    PeelGraph g{n, n_layers, entries, node_ptr, adj, deg0, n + 1};
     for (uint32_t c0 = 0; c0 < n_layers; c0 += cols) {
         const uint32_t nc = n_layers - c0 < cols ? n_layers - c0 : cols;
         PeelStats st;
-        FC_TRY(peel_run(g, c0, nc, table, ws, PEEL_SCRATCH_BYTES, s, &st, false, false));
+        FC_TRY(peel_run(g, c0, nc, table, ws, PEEL_SCRATCH_BYTES, s, &st, false, late));
     }
     return FC_OK;
 }

@@ -207,11 +207,20 @@ struct fc_server {
     // make room are released here, under the lock, so that no other lane can
     // take one of them meanwhile; their last work has completed (every batch
     // ends with a stream synchronize), so the release does not wait.
-    int admit(Request* r, uint64_t* used, const std::set<fc_graph*>& taken, uint64_t* reserve) {
+    int admit(Request* r, uint64_t* used, const std::set<fc_graph*>& taken, uint64_t* reserve,
+              bool* lean) {
         fc_graph* g = r->g;
         const uint64_t gb = fc::graph_bytes(g);
-        const uint64_t wb = plain ? fc::peel_ws_bytes(g->n, g->L, g->total_entries(), 1)
-                                  : fc::batch_peel_ws_bytes(&g, 1);
+        // a request whose scratch only fits without the peel's late form runs
+        // without it
+        auto scratch = [&](bool late) {
+            return plain ? fc::plain_peel_ws_bytes(g, late) : fc::batch_peel_ws_bytes(&g, 1, late);
+        };
+        uint64_t wb = scratch(true);
+        if (gb + wb > budget) {
+            wb = scratch(false);
+            *lean = true;
+        }
         if (gb + wb > budget) {
             finish(r, FC_ERR_BUDGET);
             cv_done.notify_all();
@@ -242,6 +251,7 @@ struct fc_server {
         uint64_t reserve = 0;  // bytes: scratch and copies not yet resident
         uint32_t sms = 0;      // SMs the peel grid may cover (0 = all)
         bool heavy = false;
+        bool lean = false;     // a graph's scratch fits only without the late form
     };
 
     // Takes the requests of the next batch out of `pending` (under mu).
@@ -278,7 +288,7 @@ struct fc_server {
         if (waiting_heavy && free_sms >= heavy_sms &&
             running_requests < max_inflight) {
             Request* h = waiting_heavy;
-            const int a = admit(h, &used, taken, &p->reserve);
+            const int a = admit(h, &used, taken, &p->reserve, &p->lean);
             if (a == 1) {
                 pending.erase(std::find(pending.begin(), pending.end(), h));
                 return;  // rejected; the lane looks again
@@ -319,7 +329,7 @@ struct fc_server {
             if (p->graphs.size() >= max_batch_graphs ||
                 running_requests + p->reqs.size() >= max_inflight)
                 break;
-            const int a = admit(r, &used, taken, &p->reserve);
+            const int a = admit(r, &used, taken, &p->reserve, &p->lean);
             if (a == 1) {
                 it = pending.erase(it);
                 continue;
@@ -349,9 +359,10 @@ struct fc_server {
         if (plain) {
             double ms = 0;
             uint32_t launches = 0, levels = 0;
-            FC_TRY(fc::batch_plain_one(graphs[0], s, &ms, &launches, &levels));
+            FC_TRY(fc::batch_plain_one(graphs[0], s, &ms, &launches, &levels, !p.lean));
         } else {
-            FC_TRY(fc::batch_peel(graphs.data(), (uint32_t)graphs.size(), &bopt, p.sms, nullptr, s));
+            FC_TRY(fc::batch_peel(graphs.data(), (uint32_t)graphs.size(), &bopt, p.sms, nullptr, s,
+                                  !p.lean));
         }
         // densest: every request's beta, one pass per graph
         for (fc_graph* g : graphs) {

@@ -1,0 +1,80 @@
+"""The peel's three single-graph forms and the hand-overs between them, at the
+sizes where they can go wrong: column counts around the words that hold four
+columns and the segments that hold 28, rows around the 64-entry items, the
+128-entry pieces and the 256-entry chunks, degrees past 16 bits, and a late
+queue too short for the run.  Every table must be the oracle's, entry for
+entry.
+
+FC_PEEL_WHOLE=0 keeps a graph off the one-block and one-cluster forms;
+FC_PEEL_LATE is the number of nodes at which the late form takes over (0:
+never); FC_PEEL_LATE_ITEMS shortens its queues."""
+import numpy as np
+import pytest
+
+import oracle as O
+from pargridcpu_b200 import MultilayerGraph, batch_run, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def check(layers, monkeypatch, **env):
+    for k, v in env.items():
+        monkeypatch.setenv(k, str(v))
+    ref = O.OracleGraph(layers).coreindex()
+    assert np.array_equal(MultilayerGraph.from_pairs(layers).coreindex(), ref)
+
+
+def graph(n, L, m, seed, gamma=2.3):
+    return synth.chung_lu_graph(n, L, m, gamma, 0.4, seed).layers
+
+
+@pytest.mark.parametrize("L", [1, 2, 3, 4, 5, 8, 9, 27, 28, 29, 57])
+@pytest.mark.parametrize("late", [0, 700, 262144])
+def test_columns_around_words_and_segments(L, late, monkeypatch):
+    check(graph(1500, L, 3000, 60 + L), monkeypatch, FC_PEEL_WHOLE=0, FC_PEEL_LATE=late)
+
+
+def spokes(lengths, seed):
+    """Hubs with rows of exactly these lengths in one layer, over a denser
+    second layer that keeps the spokes alive for some levels."""
+    n = len(lengths) + max(lengths)
+    star = [np.stack([np.full(k, i), len(lengths) + np.arange(k)], 1)
+            for i, k in enumerate(lengths)]
+    rng = np.random.default_rng(seed)
+    more = rng.integers(0, n, (6 * n, 2))
+    return [np.concatenate(star).astype(np.uint32), more[more[:, 0] != more[:, 1]].astype(np.uint32)]
+
+
+@pytest.mark.parametrize("late", [0, 300, 262144])
+def test_rows_around_items_and_chunks(late, monkeypatch):
+    layers = spokes([1, 31, 32, 33, 63, 64, 65, 127, 128, 129, 255, 256, 257, 511, 512, 513, 640,
+                     4095, 4096, 4097], 5)
+    check(layers, monkeypatch, FC_PEEL_WHOLE=0, FC_PEEL_LATE=late)
+
+
+@pytest.mark.parametrize("late", [0, 40_000, 262144])
+@pytest.mark.parametrize("leaves", [65_534, 65_535, 65_536, 70_001])
+def test_degrees_past_sixteen_bits(leaves, late, monkeypatch):
+    star = np.stack([np.zeros(leaves, np.int64), 1 + np.arange(leaves)], 1).astype(np.uint32)
+    layers = [star] + graph(leaves, 2, 2 * leaves, 17)
+    check(layers, monkeypatch, FC_PEEL_LATE=late)
+
+
+@pytest.mark.parametrize("items", [1, 200])
+def test_late_queue_too_short(items, monkeypatch):
+    check(graph(4000, 6, 16_000, 23), monkeypatch, FC_PEEL_WHOLE=0, FC_PEEL_LATE_ITEMS=items)
+
+
+@pytest.mark.parametrize("blocks", [4, 8, 16])
+def test_cluster_sizes(blocks, monkeypatch):
+    check(graph(14_000, 10, 30_000, 29), monkeypatch, FC_PEEL_CLUSTER=blocks)
+
+
+@pytest.mark.parametrize("late", [0, 900, 262144])
+def test_batch_with_one_layer_and_many_layer_graphs(late, monkeypatch):
+    monkeypatch.setenv("FC_PEEL_LATE", str(late))
+    inputs = [graph(700, 1, 2000, 31), graph(900, 30, 1500, 32), graph(1200, 4, 6000, 33),
+              graph(300, 1, 500, 34)]
+    tables, _, _ = batch_run([MultilayerGraph.from_pairs(x) for x in inputs])
+    for layers, table in zip(inputs, tables):
+        assert np.array_equal(table, O.OracleGraph(layers).coreindex())
