@@ -38,7 +38,7 @@ struct DensState {
     uint64_t hwords = 0, nwords = 0, ncells = 0;
     uint32_t* H = nullptr;             // hwords: edge histogram -> suffix sums e2
     uint32_t* N = nullptr;             // nwords: node histogram -> suffix sums |C|
-    uint32_t* coreT = nullptr;         // n*L node-major copy of the table
+    uint4* rows = nullptr;             // the table as rows of 16-bit cores (k_core_rows)
     uint64_t* d_hbase = nullptr;       // device copies of the bases (L each)
     uint64_t* d_nbase = nullptr;
     uint32_t* d_kmax = nullptr;
@@ -69,7 +69,7 @@ void free_densest_state(DeviceGraph* d, cudaStream_t st) {
     if (!s) return;
     // called with the graph's work finished (release_device waits for it, or
     // its caller knows that it has completed)
-    for (void* p : {(void*)s->H, (void*)s->N, (void*)s->coreT, (void*)s->d_hbase,
+    for (void* p : {(void*)s->H, (void*)s->N, (void*)s->rows, (void*)s->d_hbase,
                     (void*)s->d_nbase, (void*)s->d_kmax, (void*)s->cells, (void*)s->powl,
                     (void*)s->d_res, (void*)s->cell_lk})
         dev_free(p, st);
@@ -91,34 +91,42 @@ __global__ void k_colmax(const uint32_t* __restrict__ table, uint32_t n, uint32_
     if ((threadIdx.x & 31) == 0 && m) atomicMax(kmax + lam, m);
 }
 
-// L < 32: one node per thread; each of its L loads is coalesced across the
-// warp, and its values are stored as one row (a 16-byte store for L = 4)
-__global__ void k_transpose_rows(const uint32_t* __restrict__ table, uint32_t n, uint32_t L,
-                                 uint32_t* __restrict__ coreT) {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-        if (L == 4) {
-            const uint4 q = make_uint4(table[v], table[(uint64_t)n + v], table[2ull * n + v],
-                                       table[3ull * n + v]);
-            *(uint4*)(coreT + 4ull * v) = q;
-        } else {
-            for (uint32_t l = 0; l < L; l++) coreT[(uint64_t)v * L + l] = table[(uint64_t)l * n + v];
-        }
+// A word of a core row: eight columns, or four where there are no more (2.5M
+// nodes x 4 layers: 0.2 ms less than with eight).
+template <bool WIDE>
+struct CoreWord {
+    static __device__ __forceinline__ uint4 load(const uint4* rows, uint64_t i) { return rows[i]; }
+    static __device__ __forceinline__ void store(uint4* rows, uint64_t i, uint4 w) { rows[i] = w; }
+};
+template <>
+struct CoreWord<false> {
+    static __device__ __forceinline__ uint4 load(const uint4* rows, uint64_t i) {
+        const uint2 w = ((const uint2*)rows)[i];
+        return make_uint4(w.x, w.y, 0, 0);
     }
-}
+    static __device__ __forceinline__ void store(uint4* rows, uint64_t i, uint4 w) {
+        ((uint2*)rows)[i] = make_uint2(w.x, w.y);
+    }
+};
 
-__global__ void k_transpose(const uint32_t* __restrict__ table, uint32_t n, uint32_t L,
-                            uint32_t* __restrict__ coreT) {
-    // 32x32 tiles through shared memory
-    __shared__ uint32_t tile[32][33];
-    const uint32_t v0 = blockIdx.x * 32, l0 = blockIdx.y * 32;
-    for (uint32_t r = threadIdx.y; r < 32; r += blockDim.y) {
-        uint32_t l = l0 + r, v = v0 + threadIdx.x;
-        if (l < L && v < n) tile[r][threadIdx.x] = table[(uint64_t)l * n + v];
-    }
-    __syncthreads();
-    for (uint32_t r = threadIdx.y; r < 32; r += blockDim.y) {
-        uint32_t v = v0 + r, l = l0 + threadIdx.x;
-        if (l < L && v < n) coreT[(uint64_t)v * L + l] = tile[threadIdx.x][r];
+// The table as rows of 16-bit cores, a node's columns side by side, padded to
+// octets of eight (one word).  16 bits hold every core: rows have no
+// repeated entries, so a core of k takes k+1 nodes with k entries each, and a
+// graph has fewer than 2^32 entries.  Columns outside [lo, hi) are not read.
+template <bool WIDE>
+__global__ void k_core_rows(const uint32_t* __restrict__ table, uint32_t n, uint32_t lo, uint32_t hi,
+                            uint32_t octets, uint4* __restrict__ rows) {
+    const uint32_t o = blockIdx.y;
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+        uint32_t c[8];
+#pragma unroll
+        for (uint32_t i = 0; i < 8; i++) {
+            const uint32_t lam = o * 8 + i;
+            c[i] = lam >= lo && lam < hi ? table[(uint64_t)lam * n + v] : 0u;
+        }
+        CoreWord<WIDE>::store(rows, (uint64_t)v * octets + o,
+                              make_uint4(c[0] | c[1] << 16, c[2] | c[3] << 16,
+                                         c[4] | c[5] << 16, c[6] | c[7] << 16));
     }
 }
 
@@ -145,181 +153,199 @@ __global__ void k_node_hist(const uint32_t* __restrict__ table, uint32_t n,
             if (sh[i]) atomicAdd(out + i, sh[i]);
 }
 
-// Edge histogram for lambda columns [lam0, lam0 + nl).  Each warp takes a
-// contiguous slice of the entry array, 32 consecutive entries at a time (one
-// per lane), and tracks each lane's source node by advancing along node_ptr.
-// Bins live in shared memory when they fit (`sh_ok`), else in global memory.
-// The entry (v, u, l) adds one to bin (l, min(core(v), core(u))) per column.
-// The adjacency is symmetric (every (v, u, l) has its (u, v, l), in the same
-// bin), so only the entry with u > v is visited and adds two; a self-loop
-// (u = v, one entry) adds one.  The histogram is the same.
-// sh_mode: 0 the bins in global memory, 1 in shared memory as 32-bit words,
-// 2 in shared memory as 16-bit halves (a block's counts then stay below
-// 65,536: the host chooses it only when 2 x its entries per block do).
-__device__ __forceinline__ void edge_bin_add(uint32_t* sh, uint32_t* H, int sh_mode, uint32_t soff,
-                                             uint64_t hbase, uint32_t l, uint32_t km1,
-                                             uint32_t key, uint32_t cnt) {
-    if (sh_mode == 2) {
-        const uint32_t b = soff + l * km1 + key;
-        atomicAdd(sh + (b >> 1), cnt << ((b & 1) * 16));
-    } else if (sh_mode == 1) atomicAdd(sh + soff + l * km1 + key, cnt);
-    else atomicAdd(H + hbase + (uint64_t)l * km1 + key, cnt);
+// The edge histogram of groups of lambda columns.
+//
+// An edge {v, u} of layer l counts 2 in bin (l, min(core(v), core(u))) of each
+// column.  It is counted where the minimum is: entry (v, u, l) adds 2 to bin
+// (l, core(v)) when core(u) > core(v), 1 when they are equal (the entry
+// (u, v, l) adds the other 1) and 0 otherwise.  A run of entries of one (v, l)
+// then goes to one bin per column, so its counts are added up in registers and
+// each bin gets one atomic a run -- with a bin that depends on u every entry
+// needs its own, and the lanes of a warp, on one row, collide on the bin of
+// core(v).
+//
+// A warp takes a contiguous slice of the entries, 32 at a time, one a lane.
+// Eight columns are compared at once, as 16-bit halves; their counts are
+// bytes (32 entries add 64 at most), summed over a run's lanes by shuffles,
+// and the run's first lane adds them to the bins.  The bins of a group lie in
+// shared memory: as 32-bit words (mode 1), or as 16-bit halves when no block
+// can count 65,536 (mode 2); a single column whose bins do not fit has them in
+// global memory (mode 0).  All groups are one launch (blockIdx.y): a graph
+// whose entries do not fill the device once still fills it with groups.
+//
+// Bound by instruction issue (about 60 a warp and octet) and the gather of
+// the neighbours' rows.  Against an atomic per entry and column, groups one
+// after another: a pass over 220 nodes x 360 layers 2.93 -> 1.93 ms, 180,001 x
+// 17 (73M entries) 21.2 -> 19.5 ms, 2.6M x 24 (96M entries) 34.7 -> 32.8 ms.
+constexpr uint32_t EH_THREADS = 1024;
+constexpr uint32_t EH_BINS = 55 * 1024;    // 32-bit words of shared memory for bins
+constexpr uint32_t EH_MAX_COLS = 64;       // columns of a group
+constexpr uint32_t EH_MAX_GROUPS = 64;     // groups of a launch
+struct EdgeGroup {
+    uint32_t lam0, nl, bins, mode;
+};
+struct EdgeGroups {
+    EdgeGroup g[EH_MAX_GROUPS];
+};
+
+// what entries with cores u add against v, per 16-bit half: 2 above, 1 equal,
+// 0 below (v1: v - 1; halves with v = 0 are not used)
+__device__ __forceinline__ uint32_t eh_count2(uint32_t u, uint32_t v1) {
+    return __vminu2(__vmaxu2(u, v1) - v1, 0x00020002u);
+}
+__device__ __forceinline__ uint32_t eh_less1(uint32_t v) {
+    return __vmaxu2(v, 0x00010001u) - 0x00010001u;
 }
 
-// How a node's core values for the group's columns are read: one column at a
-// time (EH_SCALAR); the group is four columns starting at a multiple of four
-// with L a multiple of four, so a node's four values are one aligned 16-byte
-// load, kept across its row (EH_V4); or the group starts at a multiple of four
-// with L a multiple of four, any number of columns: four at a time, up to
-// sixteen loads issued before their values are used (EH_QUAD).
-enum : int { EH_SCALAR = 0, EH_V4 = 1, EH_QUAD = 2 };
-
-template <int MODE>
-__global__ void k_edge_hist(const uint32_t* __restrict__ node_ptr, const uint32_t* __restrict__ adj,
-                            uint32_t n, uint32_t L, uint64_t entries, FastDiv divL,
-                            const uint32_t* __restrict__ coreT, uint32_t lam0, uint32_t nl,
-                            const uint64_t* __restrict__ hbase, const uint32_t* __restrict__ kmax,
-                            uint32_t* __restrict__ H, uint32_t sh_words, int sh_ok) {
-    // sh_ok: the shared-memory mode of edge_bin_add (0, 1 or 2); sh_words:
-    // the 32-bit words the block clears
-    constexpr bool V4 = MODE == EH_V4;
+template <bool WIDE>
+__global__ void __launch_bounds__(EH_THREADS)
+k_edge_hist(const uint32_t* __restrict__ node_ptr, const uint32_t* __restrict__ adj, uint32_t n,
+            uint32_t L, uint64_t entries, FastDiv divL, const uint4* __restrict__ rows,
+            uint32_t octets, const __grid_constant__ EdgeGroups groups,
+            const uint64_t* __restrict__ hbase, const uint32_t* __restrict__ kmax,
+            uint32_t* __restrict__ H) {
     extern __shared__ uint32_t sh[];
-    __shared__ uint32_t soff[64];  // per column in the group: offset into sh
-    __shared__ uint32_t skm1[64];  // kmax + 1
-    __shared__ uint64_t shb[64];   // the column's base in H
+    __shared__ uint32_t soff[EH_MAX_COLS];  // per column of the group: offset of its bins
+    __shared__ uint32_t skm1[EH_MAX_COLS];  // kmax + 1
+    __shared__ uint64_t shb[EH_MAX_COLS];   // the column's base in H
+    const EdgeGroup gr = groups.g[blockIdx.y];
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t mode = gr.mode;
+    if (threadIdx.x < gr.nl) {
+        skm1[threadIdx.x] = kmax[gr.lam0 + threadIdx.x] + 1;
+        shb[threadIdx.x] = hbase[gr.lam0 + threadIdx.x];
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
         uint32_t o = 0;
-        for (uint32_t i = 0; i < nl; i++) {
+        for (uint32_t i = 0; i < gr.nl; i++) {
             soff[i] = o;
-            skm1[i] = kmax[lam0 + i] + 1;
-            shb[i] = hbase[lam0 + i];
             o += L * skm1[i];
         }
     }
-    if (sh_ok)
-        for (uint32_t i = threadIdx.x; i < sh_words; i += blockDim.x) sh[i] = 0;
+    if (mode) {
+        const uint32_t words = mode == 2 ? (gr.bins + 1) / 2 : gr.bins;
+        for (uint32_t i = threadIdx.x; i < words; i += EH_THREADS) sh[i] = 0;
+    }
     __syncthreads();
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    const uint64_t gw = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint64_t per = (entries + nwarps - 1) / nwarps;
-    const uint64_t e0 = gw * per, e1 = min(entries, e0 + per);
+    const uint64_t nwarps = (uint64_t)gridDim.x * (EH_THREADS / 32);
+    const uint64_t gw = (uint64_t)blockIdx.x * (EH_THREADS / 32) + (threadIdx.x >> 5);
+    const uint64_t per = ((entries + nwarps - 1) / nwarps + 31) & ~31ull;
+    const uint64_t e0 = min(entries, gw * per), e1 = min(entries, e0 + per);
+    const uint32_t o0 = gr.lam0 / 8, o1 = (gr.lam0 + gr.nl + 7) / 8;
     if (e0 < e1) {  // warp-uniform
-        // source node of this lane's first entry: last v with node_ptr[v] <= e
-        uint32_t lo = 0, hi = n;  // node_ptr[lo] <= e < node_ptr[hi]
-        if (e0 + lane < e1) {
-            while (hi - lo > 1) {
-                uint32_t mid = (lo + hi) >> 1;
-                if (node_ptr[mid] <= e0 + lane) lo = mid;
-                else hi = mid;
-            }
+        uint32_t r0 = 0, hi = n;  // the row of the slice's first entry
+        while (hi - r0 > 1) {
+            const uint32_t mid = (r0 + hi) >> 1;
+            if (node_ptr[mid] <= e0) r0 = mid;
+            else hi = mid;
         }
-        uint32_t v = lo;
-        uint32_t next_row = node_ptr[v + 1];
-        uint4 A = V4 ? *(const uint4*)(coreT + (uint64_t)v * L + lam0) : make_uint4(0, 0, 0, 0);
+        uint32_t slot = e0 + lane < e1 ? adj[e0 + lane] : 0u;
         for (uint64_t b0 = e0; b0 < e1; b0 += 32) {
-            const uint64_t e = b0 + lane;
-            uint32_t u = 0, l = 0, w = 0;  // w: what the entry adds (0, 1 or 2)
-            if (e < e1) {
-                if (next_row <= e) {
-                    do v++;
-                    while (node_ptr[v + 1] <= e);
-                    next_row = node_ptr[v + 1];
-                    if (V4) A = *(const uint4*)(coreT + (uint64_t)v * L + lam0);
-                }
-                const uint32_t slot = adj[e];
-                u = divL.div(slot);
-                l = slot - u * L;
-                w = u > v ? 2u : u == v ? 1u : 0u;
+            const bool on = b0 + lane < e1;
+            const uint32_t e = on ? (uint32_t)b0 + lane : (uint32_t)e1 - 1;
+            const uint32_t u = divL.div(slot), l = slot - u * L;
+            slot = b0 + 32 + lane < e1 ? adj[b0 + 32 + lane] : 0u;
+            // the entry's row: r0 and the row starts up to e (empty rows may
+            // make them more than a warp's worth)
+            uint32_t v = r0;
+            for (uint32_t base = r0;; base += 32) {
+                const uint32_t start = node_ptr[min(base + 1 + lane, n)];
+                uint32_t c = 0;
+#pragma unroll
+                for (uint32_t s = 16; s; s >>= 1)
+                    if (__shfl_sync(0xffffffffu, start, c + s - 1) <= e) c += s;
+                if (__shfl_sync(0xffffffffu, start, c) <= e) c++;
+                if (v == base) v += c;
+                if (!__any_sync(0xffffffffu, v == base + 32)) break;
             }
-            if (MODE == EH_QUAD) {
-                if (w) {
-                    const uint32_t* av = coreT + (uint64_t)v * L + lam0;
-                    const uint32_t* bu = coreT + (uint64_t)u * L + lam0;
-                    const uint32_t nq = nl >> 2;
-                    for (uint32_t q0 = 0; q0 < nq; q0 += 4) {
-                        uint4 qa[4], qb[4];
-#pragma unroll
-                        for (int j = 0; j < 4; j++) {
-                            qa[j] = qb[j] = make_uint4(0, 0, 0, 0);
-                            if (q0 + j < nq) {
-                                qa[j] = *(const uint4*)(av + 4 * (q0 + j));
-                                qb[j] = *(const uint4*)(bu + 4 * (q0 + j));
-                            }
-                        }
-#pragma unroll
-                        for (int j = 0; j < 4; j++) {
-                            const uint32_t i = 4 * (q0 + j);
-                            const uint32_t ka[4] = {qa[j].x, qa[j].y, qa[j].z, qa[j].w};
-                            const uint32_t kb[4] = {qb[j].x, qb[j].y, qb[j].z, qb[j].w};
-#pragma unroll
-                            for (int c = 0; c < 4; c++) {
-                                const uint32_t key = min(ka[c], kb[c]);  // 0 past nq
-                                if (key)
-                                    edge_bin_add(sh, H, sh_ok, soff[i + c], shb[i + c], l,
-                                                 skm1[i + c], key, w);
-                            }
-                        }
-                    }
-                    for (uint32_t i = nq * 4; i < nl; i++) {
-                        const uint32_t a = av[i];
-                        const uint32_t key = a ? min(a, bu[i]) : 0u;
-                        if (key) edge_bin_add(sh, H, sh_ok, soff[i], shb[i], l, skm1[i], key, w);
+            r0 = __shfl_sync(0xffffffffu, v, 31);
+            // runs of one (row, layer); `end`: the lane after the run's last
+            const uint32_t pv = __shfl_up_sync(0xffffffffu, v, 1);
+            const uint32_t pl = __shfl_up_sync(0xffffffffu, l, 1);
+            const bool head = lane == 0 || pv != v || pl != l;
+            const uint32_t heads = __ballot_sync(0xffffffffu, head);
+            const uint32_t after = heads & (0xfffffffeu << lane);
+            const uint32_t end = after ? __ffs(after) - 1 : 32u;
+            const uint32_t longest = __reduce_max_sync(0xffffffffu, head ? end - lane : 0u);
+            for (uint32_t o = o0; o < o1; o++) {
+                const uint4 a = CoreWord<WIDE>::load(rows, (uint64_t)v * octets + o);
+                const bool some = (a.x | a.y | a.z | a.w) != 0u;
+                if (!__any_sync(0xffffffffu, some)) continue;
+                uint32_t s0 = 0, s1 = 0;  // counts of columns 0-3 and 4-7, a byte each
+                if (on && some) {
+                    const uint4 b = CoreWord<WIDE>::load(rows, (uint64_t)u * octets + o);
+                    s0 = __byte_perm(eh_count2(b.x, eh_less1(a.x)), eh_count2(b.y, eh_less1(a.y)),
+                                     0x6420);
+                    s1 = __byte_perm(eh_count2(b.z, eh_less1(a.z)), eh_count2(b.w, eh_less1(a.w)),
+                                     0x6420);
+                }
+                for (uint32_t d = 1; d < longest; d <<= 1) {
+                    const uint32_t y0 = __shfl_down_sync(0xffffffffu, s0, d);
+                    const uint32_t y1 = __shfl_down_sync(0xffffffffu, s1, d);
+                    if (lane + d < end) {
+                        s0 += y0;
+                        s1 += y1;
                     }
                 }
-            } else {
-                uint4 B = make_uint4(0, 0, 0, 0);
-                if (V4 && w && (A.x | A.y | A.z | A.w))
-                    B = *(const uint4*)(coreT + (uint64_t)u * L + lam0);
-                for (uint32_t i = 0; i < nl; i++) {
-                    uint32_t a = 0, b = 0;
-                    if (V4) {
-                        a = i == 0 ? A.x : i == 1 ? A.y : i == 2 ? A.z : A.w;
-                        b = i == 0 ? B.x : i == 1 ? B.y : i == 2 ? B.z : B.w;
-                    } else if (w) {
-                        a = coreT[(uint64_t)v * L + lam0 + i];
-                        if (a) b = coreT[(uint64_t)u * L + lam0 + i];
+                if (head && some) {
+                    const uint32_t key2[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+                    for (uint32_t c = 0; c < 8; c++) {
+                        const uint32_t cnt = ((c < 4 ? s0 : s1) >> (8 * (c & 3))) & 0xFFu;
+                        const uint32_t key = (key2[c >> 1] >> (16 * (c & 1))) & 0xFFFFu;
+                        const uint32_t i = o * 8 + c - gr.lam0;  // wraps below the group
+                        if (cnt && key && i < gr.nl) {
+                            const uint32_t at = soff[i] + l * skm1[i] + key;
+                            if (mode == 1) atomicAdd(sh + at, cnt);
+                            else if (mode == 2) atomicAdd(sh + (at >> 1), cnt << ((at & 1) * 16));
+                            else atomicAdd(H + shb[i] + (uint64_t)l * skm1[i] + key, cnt);
+                        }
                     }
-                    const uint32_t key = w ? min(a, b) : 0u;
-                    if (key) edge_bin_add(sh, H, sh_ok, soff[i], shb[i], l, skm1[i], key, w);
                 }
             }
         }
     }
     __syncthreads();
-    if (sh_ok == 1) {
-        for (uint32_t i = 0; i < nl; i++) {
-            const uint32_t words = L * skm1[i];
-            uint32_t* g = H + shb[i];
-            for (uint32_t w = threadIdx.x; w < words; w += blockDim.x)
-                if (sh[soff[i] + w]) atomicAdd(g + w, sh[soff[i] + w]);
-        }
-    } else if (sh_ok == 2) {
-        for (uint32_t i = 0; i < nl; i++) {
-            const uint32_t bins = L * skm1[i];
-            uint32_t* g = H + shb[i];
-            for (uint32_t w = threadIdx.x; w < bins; w += blockDim.x) {
-                const uint32_t b = soff[i] + w;
-                const uint32_t v = (sh[b >> 1] >> ((b & 1) * 16)) & 0xFFFFu;
-                if (v) atomicAdd(g + w, v);
-            }
+    if (!mode) return;
+    for (uint32_t i = 0; i < gr.nl; i++) {
+        const uint32_t bins = L * skm1[i];
+        uint32_t* g = H + shb[i];
+        for (uint32_t w = threadIdx.x; w < bins; w += EH_THREADS) {
+            const uint32_t b = soff[i] + w;
+            const uint32_t x = mode == 1 ? sh[b] : (sh[b >> 1] >> ((b & 1) * 16)) & 0xFFFFu;
+            if (x) atomicAdd(g + w, x);
         }
     }
 }
 
-// Suffix sums over key, per (lambda, layer) row of H and per lambda of N.
+// Suffix sums over key, per (lambda, layer) row of H and per lambda of N, a
+// warp per row: 32 keys at a time from the top, summed by shuffles (a thread
+// per row pays a memory round trip per key).
 // uint32 arithmetic wraps exactly as the reference's `uint num_edge`.
-__global__ void k_suffix(uint32_t L, const uint64_t* __restrict__ hbase,
+__global__ void k_suffix(uint32_t L, uint32_t lo, uint32_t hi, const uint64_t* __restrict__ hbase,
                          const uint64_t* __restrict__ nbase, const uint32_t* __restrict__ kmax,
                          uint32_t* __restrict__ H, uint32_t* __restrict__ N) {
-    const uint32_t lam = blockIdx.x;
-    const uint32_t km1 = kmax[lam] + 1;
-    for (uint32_t l = threadIdx.x; l <= L; l += blockDim.x) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t nrows = (uint64_t)(hi - lo) * (L + 1);
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t r = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nrows; r += nwarps) {
+        const uint32_t lam = lo + (uint32_t)(r / (L + 1)), l = (uint32_t)(r % (L + 1));
+        const uint32_t km1 = kmax[lam] + 1;
         uint32_t* row = l < L ? H + hbase[lam] + (uint64_t)l * km1 : N + nbase[lam];
         uint32_t acc = 0;
-        for (int64_t k = (int64_t)km1 - 1; k >= 0; k--) {
-            acc += row[k];
-            row[k] = acc;
+        for (uint32_t done = 0; done < km1; done += 32) {
+            const bool on = done + lane < km1;
+            const uint32_t k = on ? km1 - 1 - done - lane : 0u;
+            uint32_t x = on ? row[k] : 0u;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= (uint32_t)o) x += y;
+            }
+            x += acc;
+            if (on) row[k] = x;
+            acc = __shfl_sync(0xffffffffu, x, 31);
         }
     }
 }
@@ -404,51 +430,58 @@ __global__ void k_cells(uint32_t L, uint32_t P /* pow2 >= L */, const uint64_t* 
     }
 }
 
-// The reference's preorder fold with a float running maximum.
-// One block: the cells' densities are staged in shared memory, FOLD_CHUNK at a
-// time by all threads, and thread 0 folds them in order (the float running
-// maximum is order-dependent, so the fold itself stays sequential).
-constexpr uint32_t FOLD_CHUNK = 2048;
+// The reference's preorder fold with a float running maximum: cell i wins, and
+// the maximum becomes (float)d_i, when d_i >= the maximum so far.
+//
+// The maximum after cell i is the largest (float)d_j, j <= i: rounding is
+// monotone and keeps floats, so a cell that wins raises it to its own float (or
+// leaves it), and one that does not is below it, its float too.  With F the
+// largest of all and p the first cell of float F, p wins (its float is above
+// the maximum before it), and after p exactly the cells with d_i >= F do; no
+// cell before p has d_i >= F.  So the last winner is the last cell with
+// d_i >= F, or p when there is none.  With no cell above 0, F is the initial 0
+// and the same holds.  One block: F, then both candidates.
 __global__ void k_fold(const fc_cell* __restrict__ cells, uint64_t ncells, double beta,
                        fc_densest_result* out) {
-    __shared__ double sd[FOLD_CHUNK];
-    __shared__ float s_maxd;
-    __shared__ uint64_t s_win;  // winning cell, or ~0 for none
+    __shared__ uint32_t s_max;  // floats >= 0 order like their bits
+    __shared__ unsigned long long s_first, s_last;  // p; the last cell with d >= F, plus 1
     if (threadIdx.x == 0) {
-        s_maxd = 0.0f;
-        s_win = ~0ull;
+        s_max = 0;
+        s_first = ~0ull;
+        s_last = 0;
     }
-    for (uint64_t c0 = 0; c0 < ncells; c0 += FOLD_CHUNK) {
-        const uint32_t m = ncells - c0 < FOLD_CHUNK ? (uint32_t)(ncells - c0) : FOLD_CHUNK;
-        __syncthreads();  // the last chunk is folded
-        for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) sd[i] = cells[c0 + i].density;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            float maxd = s_maxd;
-            uint64_t win = s_win;
-            for (uint32_t i = 0; i < m; i++)
-                if (sd[i] >= (double)maxd) {
-                    maxd = (float)sd[i];
-                    win = c0 + i;
-                }
-            s_maxd = maxd;
-            s_win = win;
-        }
+    __syncthreads();
+    uint32_t m = 0;
+    for (uint64_t i = threadIdx.x; i < ncells; i += blockDim.x)
+        m = max(m, __float_as_uint((float)cells[i].density));
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0) atomicMax(&s_max, m);
+    __syncthreads();
+    const float F = __uint_as_float(s_max);
+    unsigned long long first = ~0ull, last = 0;
+    for (uint64_t i = threadIdx.x; i < ncells; i += blockDim.x) {
+        const double d = cells[i].density;
+        if (first == ~0ull && (float)d == F) first = i;
+        if (d >= (double)F) last = i + 1;
     }
+    if (first != ~0ull) atomicMin(&s_first, first);
+    if (last) atomicMax(&s_last, last);
+    __syncthreads();
     if (threadIdx.x == 0) {
+        const uint64_t win = s_last ? s_last - 1 : s_first;
         fc_densest_result r;
         r.beta = beta;
         r.density = 0.0;
         r.k = r.lmd = r.length = r.lstar = 0;
-        if (s_win != ~0ull) {
-            const fc_cell c = cells[s_win];
+        if (win != ~0ull) {
+            const fc_cell c = cells[win];
             r.density = c.density;
             r.k = c.k;
             r.lmd = c.lmd;
             r.length = c.length;
             r.lstar = c.lstar;
         }
-        r.max_density_f = s_maxd;
+        r.max_density_f = F;
         r.n_cells = (uint32_t)ncells;
         *out = r;
     }
@@ -492,7 +525,8 @@ static fc_status build_hist(DeviceGraph* d, cudaStream_t st, uint32_t lo, uint32
     if (after_maxima) FC_TRY((*after_maxima)());
     d->kmax = s->kmax;
     for (uint32_t l = 0; l < L; l++)
-        if (s->kmax[l] > d->max_deg) return FC_ERR_DEVICE;  // not a valid core table
+        if (s->kmax[l] > d->max_deg || s->kmax[l] > 0xFFFFu)
+            return FC_ERR_DEVICE;  // not a valid core table
     s->hbase.assign(L, 0);
     s->nbase.assign(L, 0);
     s->cbase.assign(L, 0);
@@ -515,7 +549,8 @@ static fc_status build_hist(DeviceGraph* d, cudaStream_t st, uint32_t lo, uint32
     FC_TRY(grow(s->cell_lk, s->cell_lk_cap, 2 * nc + 2, st));
     FC_TRY(grow(s->d_hbase, s->hbase_cap, L + 1, st));
     FC_TRY(grow(s->d_nbase, s->nbase_cap, L + 1, st));
-    if (!s->coreT) FC_TRY(dev_alloc((void**)&s->coreT, (uint64_t)n * L * 4 + 4, st));
+    const uint32_t octets = (L + 7) / 8;
+    if (!s->rows) FC_TRY(dev_alloc((void**)&s->rows, (uint64_t)n * octets * 16 + 16, st));
     FC_TRY(to_device(s->d_hbase, s->hbase.data(), L * 8, st));
     FC_TRY(to_device(s->d_nbase, s->nbase.data(), L * 8, st));
     // cell list (lambda index, k) in the reference's order, for k_cells
@@ -533,84 +568,77 @@ static fc_status build_hist(DeviceGraph* d, cudaStream_t st, uint32_t lo, uint32
     FC_CUDA_TRY(cudaMemsetAsync(s->H, 0, hw * 4 + 4, st));
     FC_CUDA_TRY(cudaMemsetAsync(s->N, 0, nw * 4 + 4, st));
     if (n && L) {
-        if (L < 32) {
-            const uint32_t tb =
-                std::max<uint32_t>(1u, std::min<uint32_t>((n + 255) / 256, 8u * sm_count()));
-            k_transpose_rows<<<tb, 256, 0, st>>>(d->table, n, L, s->coreT);
-        } else {
-            dim3 tg((n + 31) / 32, (L + 31) / 32);
-            k_transpose<<<tg, dim3(32, 8), 0, st>>>(d->table, n, L, s->coreT);
-        }
+        dim3 tg(std::max<uint32_t>(1u, std::min<uint32_t>((n + 255) / 256, 8u * sm_count())), octets);
+        const bool wide = L > 4;
+        auto* const core_rows = wide ? k_core_rows<true> : k_core_rows<false>;
+        core_rows<<<tg, 256, 0, st>>>(d->table, n, lo, hi, octets, s->rows);
         FC_CUDA_TRY(cudaGetLastError());
         dim3 ng(per_col, hi - lo);
         k_node_hist<<<ng, 256, 12288 * 4, st>>>(d->table + (uint64_t)lo * n, n, s->d_nbase + lo,
                                                s->d_kmax + lo, s->N);
         count_launch(2);
         FC_CUDA_TRY(cudaGetLastError());
-        // lambda groups whose bins fit the shared-memory budget
-        const uint32_t SH_WORDS = 48 * 1024;  // 192 KB
         // once per process (thread-safe static initialisation)
-        static const cudaError_t attr_rc = cudaFuncSetAttribute(
-            k_edge_hist<EH_SCALAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, SH_WORDS * 4);
-        static const cudaError_t attr_rc4 = cudaFuncSetAttribute(
-            k_edge_hist<EH_V4>, cudaFuncAttributeMaxDynamicSharedMemorySize, SH_WORDS * 4);
-        static const cudaError_t attr_rcq = cudaFuncSetAttribute(
-            k_edge_hist<EH_QUAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, SH_WORDS * 4);
-        FC_CUDA_TRY(attr_rc);
-        FC_CUDA_TRY(attr_rc4);
-        FC_CUDA_TRY(attr_rcq);
+        static const cudaError_t attr_rc[2] = {
+            cudaFuncSetAttribute(k_edge_hist<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 EH_BINS * 4),
+            cudaFuncSetAttribute(k_edge_hist<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 EH_BINS * 4)};
+        FC_CUDA_TRY(attr_rc[wide]);
+        auto* const edge_hist = wide ? k_edge_hist<true> : k_edge_hist<false>;
         FastDiv divL;
         divL.init(L);
-        // about 16K entries per block, at most one block per SM: a block
-        // clears and flushes all of its group's bins, which small graphs
-        // should not pay on every SM (and graphs searched on other streams
-        // get the SMs this one leaves)
-        const uint64_t want = (d->entries + 16383) / 16384;
-        const int blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>(sm_count(), want));
+        // Blocks: one per 4096 entries, at most two per SM (they share an SM
+        // where the bins leave room for two: 180,001 nodes x 17 layers 0.4 ms
+        // less than one).  With many groups the groups fill the device, and a
+        // block clears and flushes its group's bins: then one per 16,384
+        // entries (220 nodes x 360 layers, 610K entries: 1.94 ms a pass with
+        // 16,384 and 2.00 with 4096; one group of 280K entries: 0.38 and 0.36).
+        const uint64_t most = 2ull * sm_count();
+        const uint64_t few = std::max<uint64_t>(
+            1, std::min<uint64_t>(most, (d->entries + 16383) / 16384));
+        const uint64_t many = std::max<uint64_t>(
+            1, std::min<uint64_t>(most, (d->entries + 4095) / 4096));
         // 16-bit bins when no block can count 65,536 in one bin (each entry
-        // adds at most 2; a block's warps take at most 32 entries more than
-        // an even share): twice the columns per pass over the entries
-        const bool half = 2 * ((d->entries + blocks - 1) / blocks + 32) < 65536;
-        const uint32_t budget = half ? 2 * SH_WORDS : SH_WORDS;  // bins
-        uint32_t lam = lo;
-        while (lam < hi) {
-            uint32_t words = 0, nl = 0;  // words: bins of the group
-            while (lam + nl < hi && nl < 64) {
-                uint32_t w = L * (s->kmax[lam + nl] + 1);
-                if (nl > 0 && words + w > budget) break;
-                words += w;
+        // adds at most 2): twice the columns per pass over the entries
+        const uint64_t warps = few * (EH_THREADS / 32);
+        const bool half =
+            2 * ((d->entries + warps - 1) / warps + 31) * (EH_THREADS / 32) < 65536;
+        const uint32_t budget = half ? 2 * EH_BINS : EH_BINS;  // bins
+        EdgeGroups groups;
+        uint32_t ng_e = 0, lam = lo;
+        size_t shb = 0;
+        while (lam < hi && d->entries) {
+            uint64_t bins = 0;
+            uint32_t nl = 0;
+            while (lam + nl < hi && nl < EH_MAX_COLS) {
+                const uint64_t w = (uint64_t)L * (s->kmax[lam + nl] + 1);
+                if (nl > 0 && bins + w > budget) break;
+                bins += w;
                 nl++;
             }
-            // with L a multiple of four, groups of a multiple of four columns
-            // keep the next group 16-byte aligned for quad loads
-            if (L % 4 == 0 && lam % 4 == 0 && nl > 4 && lam + nl < hi && nl % 4) {
-                nl &= ~3u;
-                words = 0;
-                for (uint32_t i = 0; i < nl; i++) words += L * (s->kmax[lam + i] + 1);
-            }
-            const int sh_ok = words > budget ? 0 : half ? 2 : 1;
-            if (sh_ok == 2) words = (words + 1) / 2;  // the 32-bit words cleared
-            size_t shb = sh_ok ? (size_t)words * 4 : 0;
-            if (d->entries) {
-                const bool aligned = L % 4 == 0 && lam % 4 == 0;
-                if (aligned && nl == 4)
-                    k_edge_hist<EH_V4><<<blocks, 1024, shb, st>>>(
-                        d->node_ptr, d->adj, n, L, d->entries, divL, s->coreT, lam, nl, s->d_hbase,
-                        s->d_kmax, s->H, words, sh_ok);
-                else if (aligned && nl > 4)
-                    k_edge_hist<EH_QUAD><<<blocks, 1024, shb, st>>>(
-                        d->node_ptr, d->adj, n, L, d->entries, divL, s->coreT, lam, nl, s->d_hbase,
-                        s->d_kmax, s->H, words, sh_ok);
-                else
-                    k_edge_hist<EH_SCALAR><<<blocks, 1024, shb, st>>>(
-                        d->node_ptr, d->adj, n, L, d->entries, divL, s->coreT, lam, nl, s->d_hbase,
-                        s->d_kmax, s->H, words, sh_ok);
-                count_launch();
-            }
-            FC_CUDA_TRY(cudaGetLastError());
+            EdgeGroup& gr = groups.g[ng_e++];
+            gr.lam0 = lam;
+            gr.nl = nl;
+            gr.bins = (uint32_t)std::min<uint64_t>(bins, budget + 1);
+            gr.mode = bins > budget ? 0 : half ? 2 : 1;
+            if (gr.mode) shb = std::max(shb, 4 * (size_t)(half ? (bins + 1) / 2 : bins));
             lam += nl;
+            if (ng_e == EH_MAX_GROUPS || lam >= hi) {
+                const uint32_t blocks =
+                    (uint32_t)std::max(few, std::min(many, most / ng_e));
+                edge_hist<<<dim3(blocks, ng_e), EH_THREADS, shb, st>>>(
+                    d->node_ptr, d->adj, n, L, d->entries, divL, s->rows, octets, groups,
+                    s->d_hbase, s->d_kmax, s->H);
+                count_launch();
+                FC_CUDA_TRY(cudaGetLastError());
+                ng_e = 0;
+                shb = 0;
+            }
         }
-        k_suffix<<<L, 128, 0, st>>>(L, s->d_hbase, s->d_nbase, s->d_kmax, s->H, s->N);
+        const uint64_t srows = (uint64_t)(hi - lo) * (L + 1);
+        k_suffix<<<(uint32_t)std::min<uint64_t>((srows + 7) / 8, 8u * sm_count()), 256, 0, st>>>(
+            L, lo, hi, s->d_hbase, s->d_nbase, s->d_kmax, s->H, s->N);
         count_launch();
         FC_CUDA_TRY(cudaGetLastError());
     }
@@ -662,7 +690,7 @@ fc_status densest(fc_graph* g, const double* betas, uint32_t nb, fc_densest_resu
     if (!s->d_res) FC_TRY(dev_alloc((void**)&s->d_res, sizeof(fc_densest_result), st));
     for (uint32_t b = 0; b < nb; b++) {
         FC_TRY(score_cells(d, betas[b], st));
-        k_fold<<<1, 256, 0, st>>>(s->cells, s->ncells, betas[b], s->d_res);
+        k_fold<<<1, 1024, 0, st>>>(s->cells, s->ncells, betas[b], s->d_res);
         count_launch();
         FC_CUDA_TRY(cudaGetLastError());
         FC_TRY(to_host(res + b, s->d_res, sizeof(fc_densest_result), st));
@@ -795,12 +823,11 @@ fc_status cell_members(fc_graph* g, uint32_t k, uint32_t lmd, uint32_t* nodes, u
 void densest_preload() {
     cudaFuncAttributes a;
     cudaFuncGetAttributes(&a, k_colmax);
-    cudaFuncGetAttributes(&a, k_transpose);
-    cudaFuncGetAttributes(&a, k_transpose_rows);
+    cudaFuncGetAttributes(&a, k_core_rows<false>);
+    cudaFuncGetAttributes(&a, k_core_rows<true>);
     cudaFuncGetAttributes(&a, k_node_hist);
-    cudaFuncGetAttributes(&a, k_edge_hist<EH_SCALAR>);
-    cudaFuncGetAttributes(&a, k_edge_hist<EH_V4>);
-    cudaFuncGetAttributes(&a, k_edge_hist<EH_QUAD>);
+    cudaFuncGetAttributes(&a, k_edge_hist<false>);
+    cudaFuncGetAttributes(&a, k_edge_hist<true>);
     cudaFuncGetAttributes(&a, k_suffix);
     cudaFuncGetAttributes(&a, k_cells);
     cudaFuncGetAttributes(&a, k_fold);
