@@ -52,7 +52,12 @@ struct LateJob {
     const uint2* row;            // m: first entry, entries
     const uint2* meta;           // several segments: first degree word, Q | col0 << 8
     const uint32_t* adj;
+    // G planes of `plane` words, one per word of four columns, a node's layers
+    // side by side in each: as the higher columns empty, their planes leave L2
+    // to the others (interleaved, 180,001 nodes x 17 layers is 122 MB to the
+    // end, and a decrement a random atomic at 56 G/s instead of 125).
     u64* deg;
+    uint64_t plane;
     u64* cnt;                    // m * G
     uint32_t* M;                 // m: columns not yet expanded
     const uint32_t* x_of;
@@ -77,7 +82,7 @@ struct LateView {
 
 template <bool MULTI>
 __device__ __forceinline__ uint2 lt_meta(const LateJob& j, uint32_t i) {
-    if (!MULTI) return make_uint2(i * (j.L * j.Q), j.Q | (j.col0 << 8));
+    if (!MULTI) return make_uint2(i * j.L, j.Q | (j.col0 << 8));
     return __ldg(j.meta + i);
 }
 
@@ -216,9 +221,9 @@ __device__ __forceinline__ void lt_scan(const LateJob& j, LateBlock& sb, uint32_
         const uint32_t m4 = live && q < Q ? (m >> (4 * q)) & 15u : 0u;
         u64 c4 = 0;
         if (m4 && k < FIELD_MAX) {
-            const u64* dw = j.deg + (uint64_t)mt.x + q;
+            const u64* dw = j.deg + q * j.plane + mt.x;
 #pragma unroll 4
-            for (uint32_t l = 0; l < L; l++) c4 += geq4(dw[(uint64_t)l * Q], t2);
+            for (uint32_t l = 0; l < L; l++) c4 += geq4(dw[l], t2);
         }
         uint32_t r4 = 0;
 #pragma unroll
@@ -306,8 +311,8 @@ __device__ __forceinline__ void lt_item_run(const LateJob& j, LateBlock& sb, uin
             old[e] = 0;
             if (t.a[e] != LT_NONE) {
                 const uint2 mt = lt_meta<MULTI>(j, t.a[e] >> LT_LAYER_BITS);
-                const uint64_t w = (uint64_t)mt.x + (t.a[e] & ((1u << LT_LAYER_BITS) - 1u)) *
-                                                        (mt.y & 0xFFu) + (c >> 2);
+                const uint64_t w = (c >> 2) * j.plane + mt.x +
+                                   (t.a[e] & ((1u << LT_LAYER_BITS) - 1u));
                 old[e] = atomicSub((uint32_t*)(j.deg + w) + ((c >> 1) & 1), 1u << sh);
             }
         }
@@ -343,8 +348,8 @@ __device__ __forceinline__ void lt_item_run(const LateJob& j, LateBlock& sb, uin
                 old[e] = 0;
                 if (t.a[e] != LT_NONE) {
                     const uint2 mt = lt_meta<MULTI>(j, t.a[e] >> LT_LAYER_BITS);
-                    const uint64_t w = (uint64_t)mt.x + (t.a[e] & ((1u << LT_LAYER_BITS) - 1u)) *
-                                                            (mt.y & 0xFFu) + q;
+                    const uint64_t w =
+                        q * j.plane + mt.x + (t.a[e] & ((1u << LT_LAYER_BITS) - 1u));
                     old[e] = atomicAdd(j.deg + w, 0ull - dec);
                 }
             }
@@ -547,6 +552,7 @@ struct LateBuild {
     uint2* meta;
     uint32_t* adj;
     u64* deg;
+    uint64_t plane;
     u64* cnt;
     uint32_t* M;
     uint32_t* x_of;              // the launch index of node i
@@ -625,7 +631,7 @@ __global__ void __launch_bounds__(FB_THREADS) k_lt_rows(const __grid_constant__ 
         uint32_t id, at, wt = 0;
         const uint32_t tid = fb_scan(live ? 1u : 0u, &id, s_w);
         const uint32_t tat = fb_scan(row, &at, s_w);
-        const uint32_t twt = MULTI ? fb_scan(live ? g.L * g.Q : 0u, &wt, s_w) : 0u;
+        const uint32_t twt = MULTI ? fb_scan(live ? g.L : 0u, &wt, s_w) : 0u;
         if (threadIdx.x == 0) {
             // (when fresh, ids are launch indices: neighbours are named without a map)
             s_base[0] = b.fresh ? i0 : tid ? atomicAdd(&b.ctl->m, tid) : 0u;
@@ -660,10 +666,13 @@ __global__ void __launch_bounds__(FB_THREADS) k_lt_degrees(const __grid_constant
     for (uint32_t i = blockIdx.x * (FB_THREADS / 32) + (threadIdx.x >> 5); i < m; i += warps) {
         const SegP g = seg_load<MULTI>(j, MULTI ? b.node_seg[i] : 0u);
         const uint32_t v = b.x_of[i] - g.xbase, words = g.L * g.Q;
-        u64* const dst = b.deg + (MULTI ? (uint64_t)b.meta[i].x : (uint64_t)i * words);
+        u64* const dst = b.deg + (MULTI ? b.meta[i].x : i * g.L);
         const u64* const src = (const u64*)g.deg + (uint64_t)v * words;
-        for (uint32_t w = lane; w < words; w += 32)
-            dst[w] = b.fresh ? all4(__ldg(g.deg0 + (uint64_t)v * g.L + w / g.Q)) : src[w];
+        for (uint32_t w = lane; w < words; w += 32) {
+            const uint32_t q = g.divL.div(w), l = w - q * g.L;
+            dst[q * b.plane + l] =
+                b.fresh ? all4(__ldg(g.deg0 + (uint64_t)v * g.L + l)) : src[l * g.Q + q];
+        }
         if (lane < b.G) b.cnt[(uint64_t)i * b.G + lane] = LT_DEAD;
     }
 }
@@ -818,7 +827,8 @@ void LatePlan::init(uint64_t nx, uint64_t nodes_, uint64_t words, uint64_t entri
     o_row = take(8 * nodes);
     o_meta = take(8 * nodes);
     o_adj = take(4 * entries);
-    o_deg = take(8 * words);
+    plane = words;
+    o_deg = take(8ull * G * plane);
     o_cnt = take(8ull * G * nodes);
     o_M = take(4 * nodes);
     o_x = take(4 * nodes);
@@ -841,6 +851,7 @@ static fc_status late_launch_t(const PeelJob& pj, const LatePlan& p, char* w, cu
     b.meta = (uint2*)(w + p.o_meta);
     b.adj = (uint32_t*)(w + p.o_adj);
     b.deg = (u64*)(w + p.o_deg);
+    b.plane = p.plane;
     b.cnt = (u64*)(w + p.o_cnt);
     b.M = (uint32_t*)(w + p.o_M);
     b.x_of = (uint32_t*)(w + p.o_x);
@@ -858,6 +869,7 @@ static fc_status late_launch_t(const PeelJob& pj, const LatePlan& p, char* w, cu
     j.meta = b.meta;
     j.adj = b.adj;
     j.deg = b.deg;
+    j.plane = p.plane;
     j.cnt = b.cnt;
     j.M = b.M;
     j.x_of = b.x_of;

@@ -828,13 +828,20 @@ static uint32_t default_threads() { return env_u32("FC_PEEL_THREADS", 1024) == 5
 
 // Nodes at which late.cu takes over from the peel (FC_PEEL_LATE; 0: never; at
 // most the 2^20 an item of late.cu can name).  Its rounds have the shorter
-// chain, but it writes the rows that are left once more and its decrements
-// test fewer dead neighbours away: with few nodes the chain decides, with many
-// the copy.  180,001 nodes x 17 layers: 28.0 ms at 32,768, 26.7 at 131,072,
-// 24.8 at 262,144 (every level), no more at 524,288; 24 graphs of 60 to
-// 200,000 nodes 38.1 ms at 131,072 and 35.8 at 262,144.
-static uint64_t late_nodes() {
-    const uint64_t n = env_u32("FC_PEEL_ENDGAME", 1) ? env_u32("FC_PEEL_LATE", 262144) : 0;
+// chain, but it writes the rows that are left once more and its rows are not
+// ordered.  A graph that it can take from the first level it should, unless
+// its degrees are far more than L2 holds, where both forms wait for memory and
+// the copy is for nothing: 300,001 nodes x 10 layers 5.36 ms against 6.43 with
+// 262,144 of them, 900,000 x 13 (374 MB of degrees) 12.8 against 14.2, but
+// 600,000 x 24 (691 MB) 14.5 against 13.7.  With more nodes than it can take
+// it should start late: 2.6M x 24 33.0 ms at 262,144 and 34.7 at 2^20, 180,001
+// x 17 26.7 at 131,072 (24.8 from the first level).  With several segments the
+// peel looks up an entry's segment at each access: 24 graphs of 546,404 nodes
+// together 31.5 ms at 262,144 and 27.5 at 2^20.
+static uint64_t late_nodes(bool several, uint64_t nodes, uint64_t degree_bytes) {
+    const bool all = nodes <= (1u << 20) && degree_bytes <= (512ull << 20);
+    const uint32_t most = several || all ? 1u << 20 : 262144u;
+    const uint64_t n = env_u32("FC_PEEL_ENDGAME", 1) ? env_u32("FC_PEEL_LATE", most) : 0;
     return n < (1u << 20) ? n : (1u << 20);
 }
 
@@ -870,7 +877,14 @@ struct PeelPlan {
 };
 
 static void plan_peel(const PeelSegSpec* specs, size_t count, PeelPlan* p, bool late = false) {
-    late = late && late_nodes() && late_takes(specs, count);
+    uint64_t deg_bytes = 0, all_nodes = 0;
+    for (size_t i = 0; i < count; i++) {
+        all_nodes += specs[i].g.n;
+        deg_bytes += 8ull * specs[i].g.n * specs[i].g.L * ((specs[i].ncols + 3) / 4);
+    }
+    const uint64_t stop =
+        late_nodes(count > 1 || (count && specs[0].ncols > MAX_COLS), all_nodes, deg_bytes);
+    late = late && stop && late_takes(specs, count);
     p->pack = count && peel_packs(specs[0], late);
     uint64_t at = 0;
     auto take = [&](uint64_t bytes) {
@@ -885,8 +899,7 @@ static void plan_peel(const PeelSegSpec* specs, size_t count, PeelPlan* p, bool 
     uint64_t lt_nodes = 0, lt_words = 0, lt_entries = 0, lt_items = 0, lt_most = 0;
     for (size_t i = 0; i < count; i++)
         lt_nodes += (uint64_t)specs[i].g.n * ((specs[i].ncols + most - 1) / most);
-    const uint64_t stop = late_nodes();
-    p->late = late && stop && p->pack;
+    p->late = late && p->pack;
     uint32_t max_deg = 0;
     for (size_t i = 0; i < count; i++) max_deg = std::max(max_deg, specs[i].g.max_level);
     const bool fresh = p->late && lt_nodes <= stop && max_deg <= FIELD_MAX + 1;
@@ -918,8 +931,8 @@ static void plan_peel(const PeelSegSpec* specs, size_t count, PeelPlan* p, bool 
             // (a run that starts in the late form has no peel)
             p->o_deg.push_back(take(fresh ? 0 : (uint64_t)g.n * g.L * s.Q * word));
             p->o_cnt.push_back(take(fresh ? 0 : (uint64_t)g.n * s.Q * word));
-            lt_words += (uint64_t)g.n * g.L * s.Q;
-            lt_most = std::max<uint64_t>(lt_most, (uint64_t)g.L * s.Q);
+            lt_words += (uint64_t)g.n * g.L;
+            lt_most = std::max<uint64_t>(lt_most, g.L);
             lt_entries += g.entries;
             // A step may queue a node once per column, but rarely does: a run
             // that needs more than this is done again without the late form.

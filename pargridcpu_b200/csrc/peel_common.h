@@ -206,7 +206,7 @@ struct LateCtl {
 
 // Where the scratch of one run lies.
 struct LatePlan {
-    uint64_t nodes = 0, entries = 0, q_cap = 0, total = 0;
+    uint64_t nodes = 0, entries = 0, q_cap = 0, plane = 0, total = 0;
     uint32_t G = 1;
     bool fresh = false;
     uint64_t o_ctl = 0, o_row = 0, o_meta = 0, o_adj = 0, o_deg = 0, o_cnt = 0, o_M = 0, o_x = 0,
