@@ -107,6 +107,8 @@ struct DeviceGraph {
     // reusable scratch
     void* ws = nullptr;
     size_t ws_bytes = 0;
+    void* late_ws = nullptr;  // the late form's scratch after a peel (peel_columns)
+    size_t late_bytes = 0;
     uint64_t bytes = 0;            // CSR + table
     fc_stats stats{};              // diagnostics of the last computations
     cudaStream_t home = nullptr;   // stream that may still run work on it (nullptr: none)
@@ -172,7 +174,8 @@ uint64_t peel_ws_bytes(const PeelGraph& g, uint32_t ncols, bool late = false);
 // columns [col0, col0 + ncols) of `table` (lambda-major), scratch in `ws`;
 // allocates nothing unless `instrument` (events; a trace when FC_PEEL_TRACE)
 fc_status peel_run(const PeelGraph& g, uint32_t col0, uint32_t ncols, uint32_t* table, void* ws,
-                   size_t ws_bytes, cudaStream_t s, PeelStats* st, bool instrument, bool late = false);
+                   size_t ws_bytes, cudaStream_t s, PeelStats* st, bool instrument, bool late = false,
+                   void* late_ws = nullptr);
 
 // One segment of a batched launch: columns [col0, col0 + ncols) of graph g,
 // written to table (lambda-major, L*n).

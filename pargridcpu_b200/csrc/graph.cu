@@ -623,6 +623,7 @@ void release_device(fc_graph* g, bool wait_home) {
     dev_free(d->ptab, rs);
     dev_free(d->table, rs);
     dev_free(d->ws, rs);
+    dev_free(d->late_ws, rs);
     cudaStreamSynchronize(rs);
     cudaGetLastError();
     if (cur >= 0 && d->device != cur) cudaSetDevice(cur);
@@ -632,7 +633,7 @@ void release_device(fc_graph* g, bool wait_home) {
 
 uint64_t device_bytes(const fc_graph* g) {
     if (!g->dev) return 0;
-    return g->dev->bytes + g->dev->ws_bytes;
+    return g->dev->bytes + g->dev->ws_bytes + g->dev->late_bytes;
 }
 
 // Kernels load on first use unless loaded before, and a load may wait for
