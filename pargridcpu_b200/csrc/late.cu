@@ -302,10 +302,13 @@ __device__ __forceinline__ void lt_item_run(const LateJob& j, LateBlock& sb, uin
     uint32_t rb[4] = {0, 0, 0, 0};
     uint2 row[4];
     if (!(S & (S - 1))) {
-        // removed in one column: its field's half word is all there is to
-        // decrement and compare
-        const uint32_t c = __ffs(S) - 1, sh = (c & 1) * 16;
-        uint32_t old[4];
+        // Removed in one column: one word of a neighbour's, one field of it.
+        // The atomics take the whole word here too: other items of the round
+        // decrement several of its fields at once, and atomics of two widths
+        // on the same bytes are not atomic to each other.
+        const uint32_t c = __ffs(S) - 1, sh = (c & 3) * 16;
+        const u64 minus = 0ull - (1ull << sh);
+        u64 old[4], oc[4];
 #pragma unroll
         for (int e = 0; e < 4; e++) {
             old[e] = 0;
@@ -313,26 +316,24 @@ __device__ __forceinline__ void lt_item_run(const LateJob& j, LateBlock& sb, uin
                 const uint2 mt = lt_meta<MULTI>(j, t.a[e] >> LT_LAYER_BITS);
                 const uint64_t w = (c >> 2) * j.plane + mt.x +
                                    (t.a[e] & ((1u << LT_LAYER_BITS) - 1u));
-                old[e] = atomicSub((uint32_t*)(j.deg + w) + ((c >> 1) & 1), 1u << sh);
+                old[e] = atomicAdd(j.deg + w, minus);
             }
         }
         // (results are only looked at once all are on their way)
-        uint32_t oc[4];
         uint32_t crossed = 0;
 #pragma unroll
         for (int e = 0; e < 4; e++) {
             row[e] = make_uint2(0, 0);
-            if (t.a[e] == LT_NONE || ((old[e] >> sh) & 0xFFFFu) != k + 1) continue;
+            if (t.a[e] == LT_NONE || ((uint32_t)(old[e] >> sh) & 0xFFFFu) != k + 1) continue;
             const uint32_t u = t.a[e] >> LT_LAYER_BITS;
             crossed |= 1u << e;
             row[e] = __ldg(j.row + u);
-            oc[e] = atomicSub((uint32_t*)(j.cnt + (uint64_t)u * j.G + (c >> 2)) + ((c >> 1) & 1),
-                              1u << sh);
+            oc[e] = atomicAdd(j.cnt + (uint64_t)u * j.G + (c >> 2), minus);
         }
 #pragma unroll
         for (int e = 0; e < 4; e++)
             if ((crossed >> e) & 1u)
-                if (((oc[e] >> sh) & 0xFFFFu) ==
+                if (((uint32_t)(oc[e] >> sh) & 0xFFFFu) ==
                     (lt_meta<MULTI>(j, t.a[e] >> LT_LAYER_BITS).y >> 8) + c + 1)
                     rb[e] = S;
     } else {
