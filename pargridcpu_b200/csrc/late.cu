@@ -287,7 +287,7 @@ __device__ __forceinline__ void lt_filter(const LateJob& j, LateItem& t) {
     uint32_t m[4];
 #pragma unroll
     for (int e = 0; e < 4; e++)
-        m[e] = t.a[e] != LT_NONE ? j.M[t.a[e] >> LT_LAYER_BITS] : 0u;
+        m[e] = t.a[e] != LT_NONE ? ld_either(j.M + (t.a[e] >> LT_LAYER_BITS)) : 0u;
 #pragma unroll
     for (int e = 0; e < 4; e++)
         if (!(m[e] & t.it.y)) t.a[e] = LT_NONE;  // (no mask has LT_OWNER)

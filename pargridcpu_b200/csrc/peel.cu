@@ -384,7 +384,7 @@ __device__ __forceinline__ void visit(const PeelJob& j, const Step& st, const ui
     for (int i = 0; i < N; i++) {
         const SegP g = seg_load<MULTI>(j, seg[i]);
         xu[i] = g.xbase + g.divL.div(slot[i]);
-        m[i] = S[i] ? j.M[xu[i]] : 0u;
+        m[i] = S[i] ? ld_either(j.M + xu[i]) : 0u;
     }
     uint32_t rb[N];
     if (PACK) {
@@ -495,7 +495,7 @@ __device__ __forceinline__ void visit(const PeelJob& j, const Step& st, const ui
 // table's entries are written unless the scan has written them.
 __device__ __forceinline__ void retire(const PeelJob& j, const SegP& g, const Step& st, uint32_t x,
                                        uint32_t S, bool scanned) {
-    j.M[x] &= ~S;
+    st_either(j.M + x, ld_either(j.M + x) & ~S);  // its only writer in this step
     if (scanned) return;
     const uint32_t v = x - g.xbase;
     for (uint32_t b = S; b; b &= b - 1)

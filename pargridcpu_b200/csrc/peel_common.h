@@ -118,7 +118,17 @@ __device__ __forceinline__ uint64_t global_ns() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
-__device__ __forceinline__ uint32_t ld_l2(const uint32_t* p) { return __ldcg(p); }
+// A word that another thread may be writing in the same step, where the old
+// value will do as well as the new one: the nodes' masks, which an expansion
+// tests while their owners clear columns.  (Plain accesses would race.)
+__device__ __forceinline__ uint32_t ld_either(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void st_either(uint32_t* p, uint32_t v) {
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
 
 // ---- packed fields ----------------------------------------------------------
 

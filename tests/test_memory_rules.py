@@ -28,3 +28,11 @@ def test_late_form_decrements_whole_words():
     assert packed
     for a in packed:
         assert "uint32_t*" not in a, a
+
+
+def test_masks_are_not_read_plainly_while_owners_clear_them():
+    """An expansion tests neighbours' masks while other threads clear columns
+    in theirs."""
+    for source, name in (("peel.cu", "visit"), ("peel.cu", "retire"), ("late.cu", "lt_filter"),
+                         ("late.cu", "lt_item_run")):
+        assert "j.M[" not in body(source, name), (source, name)
