@@ -180,15 +180,15 @@ struct TuneKey {
 static std::mutex g_tune_mu;
 static std::map<TuneKey, std::pair<uint32_t, uint32_t>> g_tuned;  // -> (threads, small_row)
 
-// Launch groups: consecutive graphs whose peel scratch stays within the
-// budget (FC_BATCH_WS_MB, default 32 GiB) share one launch, unless one's
-// columns are packed and the other's are not.
+// Launch groups: consecutive graphs of one kind (peel_kind; the specs are in
+// that order) whose peel scratch stays within the budget (FC_BATCH_WS_MB,
+// default 32 GiB) share one launch.
 static void plan_groups(const std::vector<PeelSegSpec>& specs, uint64_t budget, bool late,
                         std::vector<std::pair<size_t, size_t>>* groups) {
     size_t i = 0;
     while (i < specs.size()) {
         size_t e = i + 1;
-        while (e < specs.size() && peel_packs(specs[e], late) == peel_packs(specs[i], late)) {
+        while (e < specs.size() && peel_kind(specs[e].g) == peel_kind(specs[i].g)) {
             std::vector<PeelSegSpec> trial(specs.begin() + i, specs.begin() + e + 1);
             if (peel_batch_ws_bytes(trial, late) > budget) break;
             e++;
@@ -269,6 +269,10 @@ fc_status batch_peel(fc_graph* const* gs, uint32_t count, const fc_batch_options
             entries += (uint64_t)d->entries * d->L;
         }
     }
+    // (no result depends on the graphs' order)
+    std::stable_sort(specs.begin(), specs.end(), [](const PeelSegSpec& a, const PeelSegSpec& b) {
+        return peel_kind(a.g) < peel_kind(b.g);
+    });
     const uint64_t budget = (uint64_t)env_u32b("FC_BATCH_WS_MB", 32768) << 20;
     std::vector<std::pair<size_t, size_t>> groups;
     uint64_t ws_bytes = 0;

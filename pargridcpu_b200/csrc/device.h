@@ -184,11 +184,12 @@ struct PeelSegSpec {
     uint32_t col0, ncols;
     uint32_t* table;
 };
+// What g's layers allow a launch: 0 every form, 1 all but the late form
+// (late.cu), 2 only unpacked columns.  A launch runs as its highest kind, so
+// graphs of different kinds are not launched together.
+uint32_t peel_kind(const PeelGraph& g);
 // `late`: the form that takes a peel's last levels (late.cu) may be used.  Its
 // scratch comes on top of the peel's; without it the peel runs to its end.
-// Whether a launch of such segments packs four columns' degrees in a word
-// (peel.cu); segments that do and segments that do not are not launched together.
-bool peel_packs(const PeelSegSpec& sp, bool late);
 uint64_t peel_batch_ws_bytes(const std::vector<PeelSegSpec>& specs, bool late);
 // All segments in one persistent launch (threads per block and the longest row
 // queued as one item: 0 = defaults).  With *use_graph set the launch is

@@ -46,6 +46,7 @@ constexpr uint32_t LT_NONE = 0xFFFFFFFFu;   // no entry (a node has at most 20 b
 constexpr u64 LT_DEAD = 0x4000400040004000ull;
 // an entry: neighbour << 9 | layer
 constexpr uint32_t LT_LAYER_BITS = 9;
+static_assert(LATE_MAX_LAYERS == 1u << LT_LAYER_BITS, "");
 
 struct LateJob {
     uint32_t L, Q, col0, G;      // single segment: layers, words per layer; G: count words per node
@@ -805,7 +806,7 @@ __global__ void __launch_bounds__(FL_THREADS) k_lt_fill_long(const __grid_consta
 bool late_takes(const PeelSegSpec* specs, size_t count) {
     uint64_t e = 0;
     for (size_t i = 0; i < count; i++) {
-        if (specs[i].g.L > (1u << LT_LAYER_BITS)) return false;
+        if (specs[i].g.L > LATE_MAX_LAYERS) return false;
         e += specs[i].g.entries * ((specs[i].ncols + MAX_COLS - 1) / MAX_COLS);
     }
     return e < (1ull << 32);

@@ -845,13 +845,22 @@ static uint64_t late_nodes(bool several, uint64_t nodes, uint64_t degree_bytes) 
     return n < (1u << 20) ? n : (1u << 20);
 }
 
+uint32_t peel_kind(const PeelGraph& g) {
+    return g.L > MAX_PACKED_LAYERS ? 2u : g.L > LATE_MAX_LAYERS ? 1u : 0u;
+}
+
 // Packed: four columns' degrees share a word, a step's queues and masks are
 // kept apart from those of the steps around it.  Unpacked (one column per
-// segment, 32-bit degrees, one queue): when every spec is a single column,
-// where packing would only waste the other three fields, and when a count of
-// layers does not fit a field.
-bool peel_packs(const PeelSegSpec& sp, bool late) {
-    return (sp.ncols > 1 || late) && sp.g.L <= MAX_PACKED_LAYERS;
+// segment, 32-bit degrees, one queue): when every spec is a single column and
+// no late form follows, where packing would only waste the other three fields,
+// and when a count of layers does not fit a field.
+static bool packs(const PeelSegSpec* specs, size_t count, bool late) {
+    bool several = late;
+    for (size_t i = 0; i < count; i++) {
+        if (specs[i].g.L > MAX_PACKED_LAYERS) return false;
+        several |= specs[i].ncols > 1;
+    }
+    return several;
 }
 
 // One launch over some columns of some graphs: its segments and where its
@@ -888,7 +897,7 @@ static void plan_peel(const PeelSegSpec* specs, size_t count, PeelPlan* p, bool 
     const uint64_t stop =
         late_nodes(count > 1 || (count && specs[0].ncols > MAX_COLS), all_nodes, deg_bytes);
     late = late && stop && late_takes(specs, count);
-    p->pack = count && peel_packs(specs[0], late);
+    p->pack = packs(specs, count, late);
     uint64_t at = 0;
     auto take = [&](uint64_t bytes) {
         const uint64_t o = at;

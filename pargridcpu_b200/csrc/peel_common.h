@@ -203,6 +203,8 @@ __device__ __forceinline__ SegP seg_load(const PeelJob& j, uint32_t s) {
 
 // row entries of one item
 constexpr uint32_t LATE_CHUNK = 128;
+// the layers that an entry can name
+constexpr uint32_t LATE_MAX_LAYERS = 512;
 
 struct LateCtl {
     // [step mod 3] items queued in the step (low half) and blocks that have

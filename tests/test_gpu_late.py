@@ -78,3 +78,22 @@ def test_batch_with_one_layer_and_many_layer_graphs(late, monkeypatch):
     tables, _, _ = batch_run([MultilayerGraph.from_pairs(x) for x in inputs])
     for layers, table in zip(inputs, tables):
         assert np.array_equal(table, O.OracleGraph(layers).coreindex())
+
+
+@pytest.mark.parametrize("L", [512, 513])
+def test_layers_around_what_an_entry_can_name(L, monkeypatch):
+    check(graph(40, L, 60, 70 + L), monkeypatch, FC_PEEL_WHOLE=0)
+
+
+@pytest.mark.parametrize("late", [None, 0])
+@pytest.mark.parametrize("many", [30, 513])
+@pytest.mark.parametrize("order", [1, -1])
+def test_batch_of_a_one_layer_and_a_many_layer_graph(order, many, late, monkeypatch):
+    """A graph that the late form cannot take does not take it from the others."""
+    if late is not None:
+        monkeypatch.setenv("FC_PEEL_LATE", str(late))
+    inputs = [graph(700, 1, 2000, 41), graph(40, many, 60, 42), graph(900, 5, 3000, 43)][::order]
+    tables, _, report = batch_run([MultilayerGraph.from_pairs(x) for x in inputs])
+    assert report["peel_launches"] == (2 if many > 512 else 1)
+    for layers, table in zip(inputs, tables):
+        assert np.array_equal(table, O.OracleGraph(layers).coreindex())
