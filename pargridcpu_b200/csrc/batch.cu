@@ -221,29 +221,48 @@ static fc_status run_groups(const std::vector<PeelSegSpec>& specs,
     return FC_OK;
 }
 
-uint64_t batch_peel_ws_bytes(fc_graph* const* gs, uint32_t count, bool late) {
-    std::vector<PeelSegSpec> specs;
-    for (uint32_t i = 0; i < count; i++) {
-        const fc_graph* g = gs[i];
-        if (!g->n || !g->L) continue;
-        PeelSegSpec sp{};
-        sp.g.n = g->n;
-        sp.g.L = g->L;
-        sp.g.entries = g->total_entries();
-        sp.g.max_level = g->n;  // the degrees are only known on the device
-        sp.ncols = g->L;
-        specs.push_back(sp);
-    }
-    return specs.empty() ? 0 : peel_batch_ws_bytes(specs, late);
-}
+static uint64_t batch_ws_budget() { return (uint64_t)env_u32b("FC_BATCH_WS_MB", 32768) << 20; }
 
-uint64_t plain_peel_ws_bytes(const fc_graph* g, bool late) {
+// a graph as the plans' sizes need it before it is on the device, where its
+// degrees are known
+static PeelGraph host_peel_graph(const fc_graph* g) {
     PeelGraph p{};
     p.n = g->n;
     p.L = g->L;
     p.entries = g->total_entries();
     p.max_level = g->n;
-    return peel_ws_bytes(p, 1, late);
+    p.bound = true;
+    return p;
+}
+
+// A launch's scratch is not the sum of its graphs' (the late form's planes are
+// as many as its widest graph's, and graphs that start in it alone are peeled
+// first when there are many), so it is taken of all graphs together, kind by
+// kind.  Launches of several graphs stay within the budget (plan_groups).
+uint64_t batch_peel_ws_bytes(fc_graph* const* gs, uint32_t count, bool late) {
+    std::vector<PeelSegSpec> kinds[3];
+    for (uint32_t i = 0; i < count; i++) {
+        if (!gs[i]->n || !gs[i]->L) continue;
+        PeelSegSpec sp{};
+        sp.g = host_peel_graph(gs[i]);
+        sp.ncols = sp.g.L;
+        kinds[peel_kind(sp.g)].push_back(sp);
+    }
+    uint64_t bytes = 0;
+    for (const auto& specs : kinds) {
+        if (specs.empty()) continue;
+        uint64_t b = peel_batch_ws_bytes(specs, late);
+        if (b > batch_ws_budget()) {
+            b = batch_ws_budget();
+            for (const PeelSegSpec& sp : specs) b = std::max(b, peel_batch_ws_bytes({sp}, late));
+        }
+        bytes = std::max(bytes, b);
+    }
+    return bytes;
+}
+
+uint64_t plain_peel_ws_bytes(const fc_graph* g, bool late) {
+    return peel_ws_bytes(host_peel_graph(g), 1, late);
 }
 
 fc_status batch_peel(fc_graph* const* gs, uint32_t count, const fc_batch_options* opt,
@@ -273,7 +292,7 @@ fc_status batch_peel(fc_graph* const* gs, uint32_t count, const fc_batch_options
     std::stable_sort(specs.begin(), specs.end(), [](const PeelSegSpec& a, const PeelSegSpec& b) {
         return peel_kind(a.g) < peel_kind(b.g);
     });
-    const uint64_t budget = (uint64_t)env_u32b("FC_BATCH_WS_MB", 32768) << 20;
+    const uint64_t budget = batch_ws_budget();
     std::vector<std::pair<size_t, size_t>> groups;
     uint64_t ws_bytes = 0;
     void* ws = nullptr;

@@ -168,6 +168,9 @@ struct PeelGraph {
     // ordered long rows (both null when the rows are in any order)
     const uint32_t* big_id = nullptr;
     const uint32_t* ptab = nullptr;
+    // (sizes only) max_level is an upper bound: what is computed for it must do
+    // for any smaller one
+    bool bound = false;
 };
 // scratch bytes one peel launch over `ncols` columns of g needs
 uint64_t peel_ws_bytes(const PeelGraph& g, uint32_t ncols, bool late = false);

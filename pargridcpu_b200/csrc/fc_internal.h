@@ -114,9 +114,12 @@ fc_status batch_run(fc_graph* const* gs, uint32_t count, double beta, uint32_t* 
 // each graph's table is valid on the device afterwards.  rep may be NULL.
 fc_status batch_peel(fc_graph* const* gs, uint32_t count, const fc_batch_options* opt,
                      uint32_t max_sms, fc_batch_report* rep, cudaStream_t s, bool late);
-// the peel scratch batch_peel allocates for these graphs (one launch group)
-// (`late`: with the scratch of the peel's late form, which a run can do without)
+// the most peel scratch that batch_peel allocates for these graphs (`late`:
+// with the scratch of the peel's late form, which a run can do without)
 uint64_t batch_peel_ws_bytes(fc_graph* const* gs, uint32_t count, bool late);
+// server.cpp: what its admission charges for a batch's scratch
+int batch_scratch(fc_graph* const* gs, uint32_t count, uint64_t copy, uint64_t budget, bool plain,
+                  bool* lean, uint64_t* scratch);
 // the scratch of one of g's columns (the plain form)
 uint64_t plain_peel_ws_bytes(const fc_graph* g, bool late);
 // one graph, one lambda column per launch (the plain form); table valid

@@ -879,7 +879,8 @@ struct PeelPlan {
     // little (64 MB): the whole grid decrements a few hubs, and atomics on one
     // line take turns (2.5M nodes x 4 layers, 16 hub counters: the levels that
     // remove the leaves take half the time)
-    uint32_t hub_pad() const { return hub_cap * hub_stride <= (1ull << 19) ? 32u : 1u; }
+    static constexpr uint64_t HUB_PAD_MOST = 1ull << 19;
+    uint32_t hub_pad() const { return hub_cap * hub_stride <= HUB_PAD_MOST ? 32u : 1u; }
     bool late = false;           // late.cu takes the last levels, or all of them
     bool split = false;          // late.cu's scratch is not in the workspace but at late_ws
     void* late_ws = nullptr;
@@ -913,7 +914,11 @@ static void plan_peel(const PeelSegSpec* specs, size_t count, PeelPlan* p, bool 
         lt_nodes += (uint64_t)specs[i].g.n * ((specs[i].ncols + most - 1) / most);
     p->late = late && p->pack;
     uint32_t max_deg = 0;
-    for (size_t i = 0; i < count; i++) max_deg = std::max(max_deg, specs[i].g.max_level);
+    bool bound = false;
+    for (size_t i = 0; i < count; i++) {
+        max_deg = std::max(max_deg, specs[i].g.max_level);
+        bound |= specs[i].g.bound;
+    }
     const bool fresh = p->late && lt_nodes <= stop && max_deg <= FIELD_MAX + 1;
     if (!fresh && lt_nodes > stop) lt_nodes = stop;
     for (size_t i = 0; i < count; i++) {
@@ -975,7 +980,10 @@ static void plan_peel(const PeelSegSpec* specs, size_t count, PeelPlan* p, bool 
         p->o_qc = take(8 * keep * p->qc_cap);
         if (p->hub_cap) {
             p->o_hub = take(4 * p->nx);
-            p->o_ex = take(4ull * p->hub_pad() * p->hub_cap * p->hub_stride);
+            uint64_t ex = p->hub_pad() * p->hub_cap * p->hub_stride;
+            if (bound) ex = std::max(ex, 32 * std::min(p->hub_cap * p->hub_stride,
+                                                       PeelPlan::HUB_PAD_MOST));
+            p->o_ex = take(4 * ex);
         }
     }
     if (p->late) {

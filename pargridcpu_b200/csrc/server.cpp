@@ -131,6 +131,25 @@ static uint64_t graph_bytes(const fc_graph* g) {
     return 4 * (n + 1) + 4 * e + 8 * n * L + 4 * n * L + order + (16ull << 20);
 }
 
+// The scratch of a batch of these graphs, the last of which (`copy` bytes on
+// the device) asks to join it: that of the whole batch, which is not its
+// graphs' sum.  A batch runs without the peel's late form (*lean) when one of
+// its graphs only fits the budget so.  0, or 1: the last graph alone is past
+// the budget.
+int batch_scratch(fc_graph* const* gs, uint32_t count, uint64_t copy, uint64_t budget, bool plain,
+                  bool* lean, uint64_t* scratch) {
+    fc_graph* const g = gs[count - 1];
+    auto alone = [&](bool late) {
+        return plain ? plain_peel_ws_bytes(g, late) : batch_peel_ws_bytes(&g, 1, late);
+    };
+    if (copy + alone(true) > budget) {
+        if (copy + alone(false) > budget) return 1;
+        *lean = true;
+    }
+    *scratch = plain ? alone(!*lean) : batch_peel_ws_bytes(gs, count, !*lean);
+    return 0;
+}
+
 }  // namespace fc
 
 namespace {
@@ -201,58 +220,53 @@ struct fc_server {
         return !plain && r->g->total_entries() * (uint64_t)r->g->L >= heavy_visits;
     }
 
-    // Memory admission of the graph of r, not yet in the batch (under mu):
-    // 0 = admitted (`used` and the batch's `reserve` grow), 1 = can never fit
-    // (r finished with FC_ERR_BUDGET), 2 = no room now.  Graphs released to
-    // make room are released here, under the lock, so that no other lane can
-    // take one of them meanwhile; their last work has completed (every batch
-    // ends with a stream synchronize), so the release does not wait.
-    int admit(Request* r, uint64_t* used, const std::set<fc_graph*>& taken, uint64_t* reserve,
-              bool* lean) {
-        fc_graph* g = r->g;
-        const uint64_t gb = fc::graph_bytes(g);
-        // a request whose scratch only fits without the peel's late form runs
-        // without it
-        auto scratch = [&](bool late) {
-            return plain ? fc::plain_peel_ws_bytes(g, late) : fc::batch_peel_ws_bytes(&g, 1, late);
-        };
-        uint64_t wb = scratch(true);
-        if (gb + wb > budget) {
-            wb = scratch(false);
-            *lean = true;
-        }
-        if (gb + wb > budget) {
-            finish(r, FC_ERR_BUDGET);
-            cv_done.notify_all();
-            return 1;
-        }
-        const uint64_t need = (fc::residency_has(&res, g) ? 0 : gb) + wb;
-        if (*used + need > budget) {
-            // release resident graphs that nothing running or taken uses
-            std::set<fc_graph*> keep(running_graphs);
-            keep.insert(taken.begin(), taken.end());
-            keep.insert(g);
-            auto victims = fc::residency_victims(&res, keep, *used + need - budget);
-            uint64_t freed = 0;
-            for (auto& v : victims) freed += v.second;
-            if (*used + need > budget + freed) return 2;
-            for (auto& v : victims) fc::release_device(v.first, false);
-            *used -= freed;
-            st.evictions += victims.size();
-        }
-        *used += need;
-        *reserve += need;
-        return 0;
-    }
-
     struct Plan {
         std::vector<Request*> reqs;
         std::vector<fc_graph*> graphs;
-        uint64_t reserve = 0;  // bytes: scratch and copies not yet resident
+        uint64_t copies = 0;   // bytes of its device copies that are not yet resident
+        uint64_t scratch = 0;  // bytes of its peel's scratch
         uint32_t sms = 0;      // SMs the peel grid may cover (0 = all)
         bool heavy = false;
         bool lean = false;     // a graph's scratch fits only without the late form
     };
+
+    // Memory admission of the graph of r, not yet in the batch p (under mu):
+    // 0 = admitted (`used` and the batch's bytes are updated), 1 = can never fit
+    // (r finished with FC_ERR_BUDGET), 2 = no room now.  Graphs released to
+    // make room are released here, under the lock, so that no other lane can
+    // take one of them meanwhile; their last work has completed (every batch
+    // ends with a stream synchronize), so the release does not wait.
+    int admit(Request* r, uint64_t* used, Plan* p) {
+        fc_graph* g = r->g;
+        const uint64_t gb = fc::graph_bytes(g);
+        std::vector<fc_graph*> gs(p->graphs);
+        gs.push_back(g);
+        uint64_t wb = 0;
+        if (fc::batch_scratch(gs.data(), (uint32_t)gs.size(), gb, budget, plain, &p->lean, &wb)) {
+            finish(r, FC_ERR_BUDGET);
+            cv_done.notify_all();
+            return 1;
+        }
+        const uint64_t copy = fc::residency_has(&res, g) ? 0 : gb;
+        uint64_t after = *used - p->scratch + copy + wb;
+        if (after > budget) {
+            // release resident graphs that nothing running or taken uses
+            std::set<fc_graph*> keep(running_graphs);
+            keep.insert(p->graphs.begin(), p->graphs.end());
+            keep.insert(g);
+            auto victims = fc::residency_victims(&res, keep, after - budget);
+            uint64_t freed = 0;
+            for (auto& v : victims) freed += v.second;
+            if (after > budget + freed) return 2;
+            for (auto& v : victims) fc::release_device(v.first, false);
+            after -= freed;
+            st.evictions += victims.size();
+        }
+        *used = after;
+        p->copies += copy;
+        p->scratch = wb;
+        return 0;
+    }
 
     // Takes the requests of the next batch out of `pending` (under mu).
     //   * While few requests wait (fewer than backlog_requests, and not so
@@ -288,7 +302,7 @@ struct fc_server {
         if (waiting_heavy && free_sms >= heavy_sms &&
             running_requests < max_inflight) {
             Request* h = waiting_heavy;
-            const int a = admit(h, &used, taken, &p->reserve, &p->lean);
+            const int a = admit(h, &used, p);
             if (a == 1) {
                 pending.erase(std::find(pending.begin(), pending.end(), h));
                 return;  // rejected; the lane looks again
@@ -329,7 +343,7 @@ struct fc_server {
             if (p->graphs.size() >= max_batch_graphs ||
                 running_requests + p->reqs.size() >= max_inflight)
                 break;
-            const int a = admit(r, &used, taken, &p->reserve, &p->lean);
+            const int a = admit(r, &used, p);
             if (a == 1) {
                 it = pending.erase(it);
                 continue;
@@ -421,7 +435,7 @@ struct fc_server {
                 }
                 if (p.reqs.empty()) break;  // stopped and nothing pending
                 for (fc_graph* g : p.graphs) running_graphs.insert(g);
-                running_bytes += p.reserve;
+                running_bytes += p.copies + p.scratch;
                 running_requests += (uint32_t)p.reqs.size();
                 if (!plain) free_sms -= p.sms;
                 if (p.heavy) {
@@ -449,7 +463,7 @@ struct fc_server {
                 clock_advance();
                 running_lanes--;
                 for (fc_graph* g : p.graphs) running_graphs.erase(g);
-                running_bytes -= p.reserve;
+                running_bytes -= p.copies + p.scratch;
                 running_requests -= (uint32_t)p.reqs.size();
                 if (!plain) free_sms += p.sms;
                 if (p.heavy) heavy_running = false;

@@ -3,6 +3,7 @@ asked of the library itself by a small program (tests/native/plan_check.cpp)."""
 import os
 import subprocess
 
+import numpy as np
 import pytest
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -41,3 +42,40 @@ def test_packing_does_not_depend_on_which_graph_is_first(plan, env):
     alone = plan("scratch", late, 4 * [MANY_LAYERS], **env)[0]
     assert abs(first - last) <= 64 << 10  # places are rounded to 256 bytes
     assert first < 1.1 * alone
+
+
+MIXES = {
+    # a launch's planes are as many as its widest graph's
+    "wide_beside_hubs": [(2_000_000, 12, 40_000_000, 100_000), (2000, 24, 60_000, 200)],
+    "wide_beside_two_million": [(2_000_000, 4, 40_000_000, 5000), (2000, 24, 60_000, 200)],
+    "wide_beside_small": 4 * [(60_000, 4, 1_000_000, 900)] + [(2000, 24, 60_000, 200)],
+    "wide_beside_many": 15 * [(60_000, 4, 1_000_000, 900)] + [(1000, 28, 60_000, 200)],
+    # graphs that alone start in the late form, more nodes than it takes
+    "past_its_nodes": 32 * [(60_000, 12, 3_000_000, 900)],
+    "one_layer_first": [(1000, 1, 6000, 90)] + 12 * [MANY_LAYERS],
+    "many_layers_between": [(900, 6, 9000, 50), (50, 600, 60_000, 40), (900, 6, 9000, 50)],
+    # counters of hubs on lines of their own, or not, as the degrees turn out
+    "hubs_unknown": [(70_000, 28, 40_000_000, 69_000), (70_000, 4, 9_000_000, 60_000)],
+}
+
+
+@pytest.mark.parametrize("name", sorted(MIXES))
+def test_admission_charges_what_a_batch_takes(plan, name):
+    """A server charges a batch's scratch before the graphs are on the device,
+    where their degrees are known: it must cover what the launches then take."""
+    charged, lean, taken, joined = plan("admit", 150 * 10**9, MIXES[name])
+    assert not lean and joined == len(MIXES[name])
+    assert charged >= taken
+
+
+@pytest.mark.parametrize("seed", range(6))
+def test_admission_charges_what_a_random_batch_takes(plan, seed):
+    rng = np.random.default_rng(seed)
+    mix = []
+    for _ in range(int(rng.integers(2, 20))):
+        n = int(10 ** rng.uniform(2, 6.2))
+        L = int(rng.integers(1, 30))
+        entries = int(n * L * rng.uniform(0.5, 20))
+        mix.append((n, L, entries, int(rng.uniform(0, 1) ** 3 * (n - 1))))
+    charged, _, taken, joined = plan("admit", 150 * 10**9, mix)
+    assert charged >= taken and joined == len(mix)
