@@ -133,20 +133,22 @@ static uint64_t graph_bytes(const fc_graph* g) {
 
 // The scratch of a batch of these graphs, the last of which (`copy` bytes on
 // the device) asks to join it: that of the whole batch, which is not its
-// graphs' sum.  A batch runs without the peel's late form (*lean) when one of
-// its graphs only fits the budget so.  0, or 1: the last graph alone is past
-// the budget.
+// graphs' sum.  A batch whose first graph only fits the budget without the
+// peel's late form runs without it (*lean); such graphs and others do not run
+// together, so that the others keep it.  0: *scratch and *lean are the batch's
+// with this graph, 1: the last graph alone is past the budget, 2: it does not
+// go with these.
 int batch_scratch(fc_graph* const* gs, uint32_t count, uint64_t copy, uint64_t budget, bool plain,
                   bool* lean, uint64_t* scratch) {
     fc_graph* const g = gs[count - 1];
     auto alone = [&](bool late) {
         return plain ? plain_peel_ws_bytes(g, late) : batch_peel_ws_bytes(&g, 1, late);
     };
-    if (copy + alone(true) > budget) {
-        if (copy + alone(false) > budget) return 1;
-        *lean = true;
-    }
-    *scratch = plain ? alone(!*lean) : batch_peel_ws_bytes(gs, count, !*lean);
+    const bool l = copy + alone(true) > budget;
+    if (l && copy + alone(false) > budget) return 1;
+    if (count > 1 && l != *lean) return 2;
+    *lean = l;
+    *scratch = plain ? alone(!l) : batch_peel_ws_bytes(gs, count, !l);
     return 0;
 }
 
@@ -227,12 +229,12 @@ struct fc_server {
         uint64_t scratch = 0;  // bytes of its peel's scratch
         uint32_t sms = 0;      // SMs the peel grid may cover (0 = all)
         bool heavy = false;
-        bool lean = false;     // a graph's scratch fits only without the late form
+        bool lean = false;     // its scratch fits only without the late form
     };
 
     // Memory admission of the graph of r, not yet in the batch p (under mu):
     // 0 = admitted (`used` and the batch's bytes are updated), 1 = can never fit
-    // (r finished with FC_ERR_BUDGET), 2 = no room now.  Graphs released to
+    // (r finished with FC_ERR_BUDGET), 2 = not now: no room, or not with p.  Graphs released to
     // make room are released here, under the lock, so that no other lane can
     // take one of them meanwhile; their last work has completed (every batch
     // ends with a stream synchronize), so the release does not wait.
@@ -242,11 +244,14 @@ struct fc_server {
         std::vector<fc_graph*> gs(p->graphs);
         gs.push_back(g);
         uint64_t wb = 0;
-        if (fc::batch_scratch(gs.data(), (uint32_t)gs.size(), gb, budget, plain, &p->lean, &wb)) {
+        bool lean = p->lean;
+        const int a =
+            fc::batch_scratch(gs.data(), (uint32_t)gs.size(), gb, budget, plain, &lean, &wb);
+        if (a == 1) {
             finish(r, FC_ERR_BUDGET);
             cv_done.notify_all();
-            return 1;
         }
+        if (a) return a;
         const uint64_t copy = fc::residency_has(&res, g) ? 0 : gb;
         uint64_t after = *used - p->scratch + copy + wb;
         if (after > budget) {
@@ -265,6 +270,7 @@ struct fc_server {
         *used = after;
         p->copies += copy;
         p->scratch = wb;
+        p->lean = lean;
         return 0;
     }
 

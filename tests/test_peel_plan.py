@@ -79,3 +79,19 @@ def test_admission_charges_what_a_random_batch_takes(plan, seed):
         mix.append((n, L, entries, int(rng.uniform(0, 1) ** 3 * (n - 1))))
     charged, _, taken, joined = plan("admit", 150 * 10**9, mix)
     assert charged >= taken and joined == len(mix)
+
+
+def test_a_request_that_does_not_fit_does_not_change_the_batch(plan):
+    """A graph that only fits the budget without the late form, and one that
+    does not fit at all, leave the late form to a batch that has begun; the
+    first goes without it when it begins one."""
+    small, large, huge = (900, 6, 9000, 50), (300_000, 12, 60_000_000, 900), \
+        (3_000_000, 12, 600_000_000, 900)
+    with_late = plan("scratch", 1, [large])[0]
+    without = plan("scratch", 0, [large])[0]
+    assert without < with_late
+    budget = (without + with_late) // 2
+    charged, lean, taken, joined = plan("admit", budget, [small, large, huge, small])
+    assert (lean, joined) == (0, 2) and charged == taken
+    charged, lean, taken, joined = plan("admit", budget, [large, small])
+    assert (lean, joined) == (1, 1) and charged >= taken
