@@ -91,6 +91,8 @@ __global__ void k_colmax(const uint32_t* __restrict__ table, uint32_t n, uint32_
     if ((threadIdx.x & 31) == 0 && m) atomicMax(kmax + lam, m);
 }
 
+uint64_t core_rows_bytes(uint64_t n, uint64_t L) { return n * (L > 4 ? (L + 7) / 8 * 16 : 8); }
+
 // A word of a core row: eight columns, or four where there are no more (2.5M
 // nodes x 4 layers: 0.2 ms less than with eight).
 template <bool WIDE>
@@ -550,7 +552,7 @@ static fc_status build_hist(DeviceGraph* d, cudaStream_t st, uint32_t lo, uint32
     FC_TRY(grow(s->d_hbase, s->hbase_cap, L + 1, st));
     FC_TRY(grow(s->d_nbase, s->nbase_cap, L + 1, st));
     const uint32_t octets = (L + 7) / 8;
-    if (!s->rows) FC_TRY(dev_alloc((void**)&s->rows, (uint64_t)n * octets * 16 + 16, st));
+    if (!s->rows) FC_TRY(dev_alloc((void**)&s->rows, core_rows_bytes(n, L) + 16, st));
     FC_TRY(to_device(s->d_hbase, s->hbase.data(), L * 8, st));
     FC_TRY(to_device(s->d_nbase, s->nbase.data(), L * 8, st));
     // cell list (lambda index, k) in the reference's order, for k_cells

@@ -335,6 +335,13 @@ fc_status ensure_ws(DeviceGraph* d, size_t bytes, cudaStream_t s) {
     return FC_OK;
 }
 
+void free_ws(DeviceGraph* d, cudaStream_t s) {
+    dev_free(d->ws, s);
+    dev_free(d->late_ws, s);
+    d->ws = d->late_ws = nullptr;
+    d->ws_bytes = d->late_bytes = 0;
+}
+
 static int num_sms() {
     static int sms = 0;
     if (!sms) {
@@ -622,8 +629,7 @@ void release_device(fc_graph* g, bool wait_home) {
     dev_free(d->big_id, rs);
     dev_free(d->ptab, rs);
     dev_free(d->table, rs);
-    dev_free(d->ws, rs);
-    dev_free(d->late_ws, rs);
+    free_ws(d, rs);
     cudaStreamSynchronize(rs);
     cudaGetLastError();
     if (cur >= 0 && d->device != cur) cudaSetDevice(cur);

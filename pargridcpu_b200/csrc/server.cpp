@@ -123,12 +123,12 @@ static std::vector<std::pair<fc_graph*, uint64_t>> residency_victims(
 
 // Device bytes of a graph's resident copy: CSR, degrees, table, the
 // ordered rows' index (at most one per ORDER_MIN_ROW + 1 entries) and the
-// densest search's per-graph state (an estimate: transposed table, the
+// densest search's per-graph state (rows of cores; an estimate for the
 // histograms and cell records).
 static uint64_t graph_bytes(const fc_graph* g) {
     const uint64_t n = g->n, L = g->L, e = g->total_entries();
     const uint64_t order = 4 * n + (e / (ORDER_MIN_ROW + 1) + 1) * BUCKETS * 4;
-    return 4 * (n + 1) + 4 * e + 8 * n * L + 4 * n * L + order + (16ull << 20);
+    return 4 * (n + 1) + 4 * e + 8 * n * L + core_rows_bytes(n, L) + order + (16ull << 20);
 }
 
 // The scratch of a batch of these graphs, the last of which (`copy` bytes on
@@ -380,6 +380,8 @@ struct fc_server {
             double ms = 0;
             uint32_t launches = 0, levels = 0;
             FC_TRY(fc::batch_plain_one(graphs[0], s, &ms, &launches, &levels, !p.lean));
+            // the batch's charge for it ends with the batch
+            fc::free_ws(graphs[0]->dev, s);
         } else {
             FC_TRY(fc::batch_peel(graphs.data(), (uint32_t)graphs.size(), &bopt, p.sms, nullptr, s,
                                   !p.lean));

@@ -164,3 +164,33 @@ def test_server_empty_graph():
     finally:
         srv.close()
     assert table.size == 0 and (res["k"], res["lmd"], res["length"]) == (0, 0, 0)
+
+
+def _pool_used():
+    """Bytes in use of the device's stream-ordered pool."""
+    from cuda.bindings import runtime as rt
+    err, pool = rt.cudaDeviceGetDefaultMemPool(0)
+    assert err == rt.cudaError_t.cudaSuccess
+    err, used = rt.cudaMemPoolGetAttribute(pool, rt.cudaMemPoolAttr.cudaMemPoolAttrUsedMemCurrent)
+    assert err == rt.cudaError_t.cudaSuccess
+    return int(used)
+
+
+@pytest.mark.parametrize("plain", [False, True])
+@pytest.mark.parametrize("layers", [1, 2])
+def test_server_resident_bytes_cover_what_graphs_keep(layers, plain):
+    """What an idle server says it keeps covers what its graphs hold on the
+    device: the densest search's rows of few layers, and no peel scratch."""
+    n = 4_000_000
+    path = np.stack([np.arange(n - 1), np.arange(1, n)], 1).astype(np.uint32)
+    g = MultilayerGraph.from_pairs([path] * layers)
+    before = _pool_used()
+    srv = Server(plain=plain, lanes=1)
+    try:
+        table, res, _ = srv.wait(srv.submit(g, 1.0), timeout_ms=120000)
+        held = _pool_used() - before
+        kept = srv.stats()["resident_bytes"]
+    finally:
+        srv.close()
+    assert np.all(table == 1) and res["length"] == n
+    assert held <= kept, (held, kept)
