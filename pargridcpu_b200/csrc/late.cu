@@ -658,7 +658,10 @@ __global__ void __launch_bounds__(FB_THREADS) k_lt_rows(const __grid_constant__ 
 }
 
 // The degree words: copied, or every column's from the full degrees; the
-// counts of the columns that no scan will look at.
+// counts of the columns that no scan will look at.  A word whose columns have
+// all left the node was perhaps never written (the first scan writes none
+// whose columns all go there): it starts with full fields, which count more
+// than the neighbours left, as the rounds' bounds ask.
 template <bool MULTI>
 __global__ void __launch_bounds__(FB_THREADS) k_lt_degrees(const __grid_constant__ PeelJob j,
                                                            const __grid_constant__ LateBuild b) {
@@ -668,12 +671,15 @@ __global__ void __launch_bounds__(FB_THREADS) k_lt_degrees(const __grid_constant
     for (uint32_t i = blockIdx.x * (FB_THREADS / 32) + (threadIdx.x >> 5); i < m; i += warps) {
         const SegP g = seg_load<MULTI>(j, MULTI ? b.node_seg[i] : 0u);
         const uint32_t v = b.x_of[i] - g.xbase, words = g.L * g.Q;
+        const uint32_t M = b.M[i];
         u64* const dst = b.deg + (MULTI ? b.meta[i].x : i * g.L);
         const u64* const src = (const u64*)g.deg + (uint64_t)v * words;
         for (uint32_t w = lane; w < words; w += 32) {
             const uint32_t q = g.divL.div(w), l = w - q * g.L;
-            dst[q * b.plane + l] =
-                b.fresh ? all4(__ldg(g.deg0 + (uint64_t)v * g.L + l)) : src[l * g.Q + q];
+            u64 d = ~0ull;
+            if (b.fresh) d = all4(__ldg(g.deg0 + (uint64_t)v * g.L + l));
+            else if ((M >> (4 * q)) & 15u) d = src[l * g.Q + q];
+            dst[q * b.plane + l] = d;
         }
         if (lane < b.G) b.cnt[(uint64_t)i * b.G + lane] = LT_DEAD;
     }

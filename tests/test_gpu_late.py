@@ -97,3 +97,16 @@ def test_batch_of_a_one_layer_and_a_many_layer_graph(order, many, late, monkeypa
     assert report["peel_launches"] == (2 if many > 512 else 1)
     for layers, table in zip(inputs, tables):
         assert np.array_equal(table, O.OracleGraph(layers).coreindex())
+
+
+def test_columns_that_leave_in_the_first_scan(monkeypatch):
+    """Nodes with edges in few of many layers lose their higher columns at
+    level 0, and with them whole words that are never written; a graph that
+    used the same scratch before leaves it with other contents."""
+    monkeypatch.setenv("FC_PEEL_WHOLE", "0")
+    monkeypatch.setenv("FC_PEEL_LATE", "3000")
+    dense = graph(4000, 12, 9000, 51)
+    few = graph(4000, 3, 16_000, 52) + graph(200, 9, 900, 53)
+    for layers in (dense, few, dense):
+        ref = O.OracleGraph(layers).coreindex()
+        assert np.array_equal(MultilayerGraph.from_pairs(layers).coreindex(), ref)

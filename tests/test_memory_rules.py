@@ -36,3 +36,11 @@ def test_masks_are_not_read_plainly_while_owners_clear_them():
     for source, name in (("peel.cu", "visit"), ("peel.cu", "retire"), ("late.cu", "lt_filter"),
                          ("late.cu", "lt_item_run")):
         assert "j.M[" not in body(source, name), (source, name)
+
+
+def test_hand_over_reads_only_written_degrees():
+    """The first scan writes no degree word whose columns all leave the node
+    there, and the scratch is not cleared: the hand-over to the late form
+    copies a word only if one of its columns is left."""
+    text = body("late.cu", "k_lt_degrees")
+    assert re.search(r"if \(\(M >> \(4 \* q\)\) & 15u\) d = src\[", text)
