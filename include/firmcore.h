@@ -247,6 +247,9 @@ fc_status fc_mlcd_query(const uint32_t* cores, uint32_t n, uint32_t P, const uin
  * fc_densest on the graph alone.  With `plain` set it runs the baseline
  * instead: one graph and one lambda column per launch, one after another. */
 typedef struct fc_batch_options {
+    /* The grid-wide peel's launch shape.  A launch of up to 2^20 nodes runs in a
+     * form that has neither parameter: they change nothing there and nothing is
+     * tuned.  No result depends on them. */
     uint32_t block_threads;    /* 512 or 1024 threads per block; 0 = autotuned */
     uint32_t hub_threshold;    /* longest row queued as one work item (longer rows are
                                   split in 256-entry pieces); 0 = autotuned */
@@ -259,8 +262,8 @@ typedef struct fc_batch_report {
     double peel_ms;            /* device time of the peel launch(es), CUDA events */
     double densest_ms;         /* time of the densest searches (they overlap on streams) */
     uint32_t peel_launches;
-    uint32_t block_threads;    /* the configuration used */
-    uint32_t hub_threshold;
+    uint32_t block_threads;    /* the grid-wide peel's configuration: given, tuned, */
+    uint32_t hub_threshold;    /*   or the defaults where no launch runs it */
     uint32_t levels;
     int used_cuda_graph;
     int autotuned;             /* 1 when this call measured the candidates */
@@ -297,8 +300,9 @@ typedef struct fc_server_options {
     uint32_t max_inflight;      /* requests on the device at once (0 = 256) */
     uint32_t lanes;             /* batches on the device at once (0 = 2) */
     uint32_t max_batch_graphs;  /* distinct graphs in one batch (0 = 64) */
-    uint32_t block_threads;     /* peel launch shape (0 = 1024 threads, */
-    uint32_t hub_threshold;     /*   rows of more than 64 entries split) */
+    uint32_t block_threads;     /* grid-wide peel's launch shape, as in */
+    uint32_t hub_threshold;     /*   fc_batch_options (0 = 1024 threads, rows of more
+                                     than 64 entries split) */
     int plain;                  /* 1 = the one-at-a-time baseline */
     uint64_t heavy_visits;      /* entries x L at which a request runs alone (0 = 1e9) */
 } fc_server_options;

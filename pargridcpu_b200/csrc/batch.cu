@@ -3,10 +3,11 @@
 // Batched form: every graph is one segment of a single persistent peel launch
 // (all its lambda columns; graphs whose scratch would not fit one launch are
 // spread over a few launches), optionally captured in a CUDA graph; then the
-// densest search per graph.  The block size and the hub threshold (longest
-// row queued as one work item) are chosen by an autotuner that times the
-// candidates on a sample of the batch and remembers the winner per batch
-// shape.  Results do not depend on either, so tuning never changes an output.
+// densest search per graph.  Where the grid-wide peel has a part in it, its
+// block size and hub threshold (longest row queued as one work item) are
+// chosen by an autotuner that times the candidates on a sample of the batch
+// and remembers the winner per batch shape.  Results do not depend on either,
+// so tuning never changes an output.
 //
 // Plain form (the baseline): one graph after another, one lambda column per
 // launch -- "a single launch per lambda".
@@ -318,7 +319,12 @@ fc_status batch_peel(fc_graph* const* gs, uint32_t count, const fc_batch_options
     uint32_t small_row = opt ? opt->hub_threshold : 0;
     bool tuned_now = false;
     fc_status rc = FC_OK;
-    if (!specs.empty() && (!threads || !small_row)) {
+    // the late form has neither parameter: nothing to tune when it takes every
+    // level of every launch
+    bool peels = false;
+    for (const auto& gr : groups)
+        peels = peels || peel_batch_peels({specs.begin() + gr.first, specs.begin() + gr.second}, late);
+    if (peels && (!threads || !small_row)) {
         TuneKey key{count, maxL, max_sms, entries >> 20};
         std::pair<uint32_t, uint32_t> best{0, 0};
         {
@@ -327,19 +333,20 @@ fc_status batch_peel(fc_graph* const* gs, uint32_t count, const fc_batch_options
             if (it != g_tuned.end()) best = it->second;
         }
         if (!best.first) {
-            // candidates timed on a sample: every k-th graph, up to 32 of them
+            // candidates timed on a sample: every k-th graph, up to 32 of them,
+            // without the late form, which would take so few from the first level
             std::vector<PeelSegSpec> sample;
             const size_t step = std::max<size_t>(1, specs.size() / 32);
             for (size_t i = 0; i < specs.size(); i += step) sample.push_back(specs[i]);
             std::vector<std::pair<size_t, size_t>> sg;
-            plan_groups(sample, ws_bytes, late, &sg);
+            plan_groups(sample, ws_bytes, false, &sg);
             double best_ms = 1e300;
             for (uint32_t th : {512u, 1024u})
                 for (uint32_t sr : {16u, 32u, 64u}) {
                     double ms;
                     uint32_t lv;
                     bool gr;
-                    rc = run_groups(sample, sg, ws, ws_bytes, s, th, sr, false, max_sms, late, &ms, &lv,
+                    rc = run_groups(sample, sg, ws, ws_bytes, s, th, sr, false, max_sms, false, &ms, &lv,
                                     &gr);
                     if (rc != FC_OK) break;
                     if (ms < best_ms) {
@@ -356,6 +363,10 @@ fc_status batch_peel(fc_graph* const* gs, uint32_t count, const fc_batch_options
         if (!threads) threads = best.first;
         if (!small_row) small_row = best.second;
     }
+    uint32_t dflt_threads, dflt_row;
+    peel_defaults(&dflt_threads, &dflt_row);
+    if (!threads) threads = dflt_threads;
+    if (!small_row) small_row = dflt_row;
     double peel_ms = 0;
     uint32_t levels = 0;
     bool graphed = false;

@@ -197,6 +197,11 @@ uint32_t peel_kind(const PeelGraph& g);
 // `late`: the form that takes a peel's last levels (late.cu) may be used.  Its
 // scratch comes on top of the peel's; without it the peel runs to its end.
 uint64_t peel_batch_ws_bytes(const std::vector<PeelSegSpec>& specs, bool late);
+// whether the grid-wide peel (peel.cu) has a part in the launch, or the late
+// form takes every level of it
+bool peel_batch_peels(const std::vector<PeelSegSpec>& specs, bool late);
+// the threads per block and the longest row queued as one item by default
+void peel_defaults(uint32_t* threads, uint32_t* small_row);
 // All segments in one persistent launch (threads per block and the longest row
 // queued as one item: 0 = defaults).  With *use_graph set the launch is
 // captured in a CUDA graph; on return *use_graph says whether it was.  The grid

@@ -1206,6 +1206,17 @@ uint64_t peel_batch_ws_bytes(const std::vector<PeelSegSpec>& specs, bool late) {
     return run_bytes(specs.data(), specs.size(), late);
 }
 
+bool peel_batch_peels(const std::vector<PeelSegSpec>& specs, bool late) {
+    PeelPlan p;
+    plan_peel(specs.data(), specs.size(), &p, late);
+    return !(p.late && p.lp.fresh);
+}
+
+void peel_defaults(uint32_t* threads, uint32_t* small_row) {
+    *threads = default_threads();
+    *small_row = env_u32("FC_PEEL_SMALL_ROW", SMALL_ROW_DEFAULT);
+}
+
 fc_status peel_batch(const std::vector<PeelSegSpec>& specs, void* ws, size_t ws_bytes,
                      cudaStream_t s, PeelStats* st, uint32_t threads, uint32_t small_row,
                      bool* use_graph, uint32_t max_sms, bool late) {

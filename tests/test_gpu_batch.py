@@ -141,3 +141,47 @@ def test_c4_mix_batched_equals_the_reference():
             nodes, _ = g.densest_members(r)
             assert hashlib.sha256(np.ascontiguousarray(nodes, dtype="<u4").tobytes()) \
                 .hexdigest() == f["nodes_sha256"], i
+
+
+def test_no_tuning_where_the_late_form_takes_every_level(monkeypatch):
+    """A batch that runs without the grid-wide peel times no candidates: its
+    first call launches what its second does.  One that does run it is tuned,
+    once."""
+    from pargridcpu_b200 import launch_count
+
+    def run(seed):
+        inputs = [synth.chung_lu_graph(900 + i, 3, 2500, 2.3, 0.3, seed + i).layers for i in range(3)]
+        launches, reports = [], []
+        for _ in range(2):
+            graphs = [MultilayerGraph.from_pairs(x) for x in inputs]
+            for g in graphs:
+                g.upload()
+            before = launch_count()
+            tables, _, report = batch_run(graphs)
+            launches.append(launch_count() - before)
+            reports.append(report)
+            for x, t in zip(inputs, tables):
+                assert np.array_equal(t, O.OracleGraph(x).coreindex())
+        return launches, reports
+
+    launches, reports = run(510)
+    assert launches[0] == launches[1]
+    assert [r["autotuned"] for r in reports] == [0, 0]
+    assert reports[0]["block_threads"] in (512, 1024) and reports[0]["hub_threshold"] > 0
+    monkeypatch.setenv("FC_PEEL_LATE", "500")
+    launches, reports = run(510)
+    assert launches[0] > launches[1]
+    assert [r["autotuned"] for r in reports] == [1, 0]
+
+
+@pytest.mark.parametrize("late", [0, 700])
+@pytest.mark.parametrize("threads,row", [(512, 16), (512, 64), (1024, 32)])
+def test_grid_wide_peel_of_a_batch_at_each_launch_shape(batch, threads, row, late, monkeypatch):
+    """With the late form held off (0: altogether) the given launch shapes run
+    over several segments."""
+    monkeypatch.setenv("FC_PEEL_LATE", str(late))
+    layers, expected = batch
+    graphs = [MultilayerGraph.from_pairs(ls) for ls in layers]
+    tables, results, report = batch_run(graphs, beta=1.0, block_threads=threads, hub_threshold=row)
+    _check(tables, results, expected)
+    assert (report["block_threads"], report["hub_threshold"]) == (threads, row)
