@@ -443,7 +443,7 @@ __device__ __forceinline__ uint32_t lt_barrier(const LateJob& j, uint64_t t_star
     LateCtl* const c = j.ctl;
     __syncthreads();
     if (threadIdx.x == 0) {
-        if (blockIdx.x == 0 && global_ns() - t_start > j.deadline_ns)
+        if (blockIdx.x == 0 && past_deadline(t_start, j.deadline_ns))
             atomicCAS(&c->err.v, PEEL_OK, PEEL_ERR_DEADLINE);
         asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(word), "l"(1ull << 32)
                      : "memory");
@@ -479,8 +479,8 @@ __global__ void __launch_bounds__(T, 1) k_late(const __grid_constant__ LateJob j
     // an error: nothing reads them
     if (j.ctl0->err.v) return;
     const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
-    const uint64_t t_start = lead ? global_ns() : 0;
-    uint64_t t_last = t_start, t_scan = 0;
+    const uint64_t t_start = lead ? j.ctl0->t_start : 0;
+    uint64_t t_last = lead ? global_ns() : 0, t_scan = 0;
     uint32_t step = 0, level = 0;
     const uint32_t k0 = c->first_level, list0 = c->list;
     uint32_t alive_n = c->m;
@@ -609,8 +609,10 @@ __global__ void __launch_bounds__(FB_THREADS) k_lt_rows(const __grid_constant__ 
     const PeelCtl* const pc = j.ctl;
     const uint32_t n_in = b.fresh ? j.nx : pc->stopped ? pc->stop_alive : 0u;
     const uint32_t* const list = b.fresh ? nullptr : j.alive[pc->stop_list & 1u];
-    if (blockIdx.x == 0 && threadIdx.x == 0)
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
         b.ctl->first_level = b.fresh ? 0u : pc->stop_level + 1;
+        b.ctl->t_start = !b.fresh ? pc->t_start : j.t_start ? j.t_start : global_ns();
+    }
     for (uint32_t i0 = blockIdx.x * FB_THREADS; i0 < n_in; i0 += gridDim.x * FB_THREADS) {
         const uint32_t i = i0 + threadIdx.x;
         uint32_t x = 0, s = 0, row = 0, v = 0, M = 0;

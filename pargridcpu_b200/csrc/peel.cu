@@ -57,7 +57,7 @@ __device__ void grid_barrier(const PeelJob& j, uint32_t& nbar, uint64_t t_start,
     __syncthreads();
     if (threadIdx.x == 0) {
         const uint32_t target = ++nbar * gridDim.x;
-        if (blockIdx.x == 0 && global_ns() - t_start > j.deadline_ns)
+        if (blockIdx.x == 0 && past_deadline(t_start, j.deadline_ns))
             atomicCAS(&c->err.v, PEEL_OK, PEEL_ERR_DEADLINE);
         red_add_release(&c->arrive.v, 1u);
         uint64_t t0 = 0;
@@ -658,8 +658,9 @@ __global__ void __launch_bounds__(T, BPS) k_peel(const __grid_constant__ PeelJob
     __shared__ StepView sv;
     PeelCtl* const c = j.ctl;
     const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
-    const uint64_t t_start = lead ? global_ns() : 0;
-    uint64_t t_last = t_start, t_scan = 0, ph0 = 0, ph1 = 0;
+    uint64_t t_last = lead ? global_ns() : 0, t_scan = 0, ph0 = 0, ph1 = 0;
+    const uint64_t t_start = j.t_start ? j.t_start : t_last;
+    if (lead) c->t_start = t_start;
     uint32_t nbar = 0, items = 0;
     uint32_t step = 0, level = 0;
     uint32_t alive_n = j.nx, pns = 0, pnc = 0;  // pns, pnc: items the last step read
@@ -1069,10 +1070,17 @@ static fc_status reset_job(const PeelJob& j, bool pack, cudaStream_t s) {
     return FC_OK;
 }
 
+// A run that needs longer queues than the late form's is done again without it,
+// as part of the same run.
+struct Again {
+    bool needed = false;
+    uint64_t t_start = 0;  // when the run began
+};
+
 // Launches the prepared job and reads its control block back.
 static fc_status run_job(PeelJob& j, const PeelPlan& p, uint32_t threads, cudaStream_t s, PeelStats* st,
-                         bool instrument, uint32_t col0, uint32_t ncols,
-                         bool* use_graph = nullptr, bool* again = nullptr) {
+                         bool instrument, uint32_t col0, uint32_t ncols, bool* use_graph,
+                         Again* again) {
     const bool pack = p.pack;
     char* const lw =
         p.split ? (char*)p.late_ws : (char*)j.ctl - p.o_ctl + p.o_late;  // late.cu's scratch
@@ -1143,8 +1151,9 @@ static fc_status run_job(PeelJob& j, const PeelPlan& p, uint32_t threads, cudaSt
         for (const LateCtl& c : lo)
             if (!out.err.v) {
                 out.err.v = c.err.v;
-                if (again) *again = c.err.v == PEEL_ERR_QUEUE;
+                again->needed = c.err.v == PEEL_ERR_QUEUE;
             }
+        again->t_start = lo[0].t_start;
         if (tracing)
             fprintf(stderr, "late-trace nodes %u entries %u first level %u levels %u\n", lo[0].m,
                     lo[0].entries, lo[0].first_level, lo[0].levels + lo[1].levels);
@@ -1187,19 +1196,28 @@ static fc_status run_job(PeelJob& j, const PeelPlan& p, uint32_t threads, cudaSt
     return FC_OK;
 }
 
-fc_status peel_run(const PeelGraph& g, uint32_t col0, uint32_t ncols, uint32_t* table, void* ws,
-                   size_t ws_bytes, cudaStream_t s, PeelStats* st, bool instrument, bool late,
-                   void* late_ws) {
+static fc_status run_from(uint64_t t_start, const PeelGraph& g, uint32_t col0, uint32_t ncols,
+                          uint32_t* table, void* ws, size_t ws_bytes, cudaStream_t s, PeelStats* st,
+                          bool instrument, bool late, void* late_ws) {
     const PeelSegSpec sp{g, col0, ncols, table};
     PeelPlan p;
     plan_peel(&sp, 1, &p, late, late_ws != nullptr);
     p.late_ws = late_ws;
     PeelJob j;
     FC_TRY(carve(p, ws, ws_bytes, s, &j));
-    bool again = false;
+    j.t_start = t_start;
+    Again again;
     const fc_status rc = run_job(j, p, default_threads(), s, st, instrument, col0, ncols, nullptr,
                                  &again);
-    return again ? peel_run(g, col0, ncols, table, ws, ws_bytes, s, st, instrument, false) : rc;
+    if (!again.needed) return rc;
+    return run_from(again.t_start, g, col0, ncols, table, ws, ws_bytes, s, st, instrument, false,
+                    nullptr);
+}
+
+fc_status peel_run(const PeelGraph& g, uint32_t col0, uint32_t ncols, uint32_t* table, void* ws,
+                   size_t ws_bytes, cudaStream_t s, PeelStats* st, bool instrument, bool late,
+                   void* late_ws) {
+    return run_from(0, g, col0, ncols, table, ws, ws_bytes, s, st, instrument, late, late_ws);
 }
 
 uint64_t peel_batch_ws_bytes(const std::vector<PeelSegSpec>& specs, bool late) {
@@ -1217,9 +1235,9 @@ void peel_defaults(uint32_t* threads, uint32_t* small_row) {
     *small_row = env_u32("FC_PEEL_SMALL_ROW", SMALL_ROW_DEFAULT);
 }
 
-fc_status peel_batch(const std::vector<PeelSegSpec>& specs, void* ws, size_t ws_bytes,
-                     cudaStream_t s, PeelStats* st, uint32_t threads, uint32_t small_row,
-                     bool* use_graph, uint32_t max_sms, bool late) {
+static fc_status batch_from(uint64_t t_start, const std::vector<PeelSegSpec>& specs, void* ws,
+                            size_t ws_bytes, cudaStream_t s, PeelStats* st, uint32_t threads,
+                            uint32_t small_row, bool* use_graph, uint32_t max_sms, bool late) {
     if (specs.empty()) return FC_OK;
     PeelPlan p;
     plan_peel(specs.data(), specs.size(), &p, late);
@@ -1227,16 +1245,24 @@ fc_status peel_batch(const std::vector<PeelSegSpec>& specs, void* ws, size_t ws_
     FC_TRY(carve(p, ws, ws_bytes, s, &j));
     j.small_row = small_row;
     j.max_sms = max_sms;
+    j.t_start = t_start;
     if (!threads) threads = default_threads();
     // the segment table must be on the device before a captured launch runs
     if (use_graph && *use_graph) FC_CUDA_TRY(cudaStreamSynchronize(s));
-    bool again = false;
+    Again again;
     const bool want_graph = use_graph && *use_graph;
     const fc_status rc =
         run_job(j, p, threads, s, st, true, specs[0].col0, specs[0].ncols, use_graph, &again);
-    if (!again) return rc;
+    if (!again.needed) return rc;
     if (use_graph) *use_graph = want_graph;
-    return peel_batch(specs, ws, ws_bytes, s, st, threads, small_row, use_graph, max_sms, false);
+    return batch_from(again.t_start, specs, ws, ws_bytes, s, st, threads, small_row, use_graph,
+                      max_sms, false);
+}
+
+fc_status peel_batch(const std::vector<PeelSegSpec>& specs, void* ws, size_t ws_bytes,
+                     cudaStream_t s, PeelStats* st, uint32_t threads, uint32_t small_row,
+                     bool* use_graph, uint32_t max_sms, bool late) {
+    return batch_from(0, specs, ws, ws_bytes, s, st, threads, small_row, use_graph, max_sms, late);
 }
 
 void peel_preload() {

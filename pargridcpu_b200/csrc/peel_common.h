@@ -49,6 +49,7 @@ struct PeelCtl {
     uint64_t ph_ns[2];  // time in scans, in expansions
     uint32_t levels, items, err_level, nhub;
     uint32_t bad_item, bad_where;  // what PEEL_ERR_ITEM saw
+    uint64_t t_start;   // when the run began (the deadline counts from there)
     // the run stopped: the nodes alive after level stop_level are in list
     // `stop_list`, stop_alive entries (some of them removed since its scan)
     uint32_t stopped, stop_level, stop_list, stop_alive;
@@ -89,7 +90,8 @@ struct PeelJob {
     uint32_t max_level;
     uint32_t small_row;   // longest row queued as one item; longer rows go in chunks
     uint64_t timeout_ns;  // longest wait at a barrier
-    uint64_t deadline_ns; // longest whole run
+    uint64_t deadline_ns; // longest whole run, all its launches together
+    uint64_t t_start;     // when it began, for a repetition; else 0 (this launch begins it)
     // optional per-level trace: {scan ns, expand ns, rounds, items, alive}
     unsigned long long* trace;
     uint32_t trace_levels;
@@ -117,6 +119,10 @@ __device__ __forceinline__ uint64_t global_ns() {
     uint64_t t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
+}
+// whether a run that began at t_start is past its deadline
+__device__ __forceinline__ bool past_deadline(uint64_t t_start, uint64_t deadline_ns) {
+    return (int64_t)(global_ns() - t_start) > (int64_t)deadline_ns;
 }
 // A word that another thread may be writing in the same step, where the old
 // value will do as well as the new one: the nodes' masks, which an expansion
@@ -214,6 +220,7 @@ struct LateCtl {
     Hot err;
     uint32_t m, first_level, list, nfill, levels;  // where it starts: nodes, level, list
     uint32_t entries, words;  // row entries and degree words reserved
+    uint64_t t_start;   // when the run began
 };
 
 // Where the scratch of one run lies.

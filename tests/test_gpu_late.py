@@ -12,7 +12,7 @@ import numpy as np
 import pytest
 
 import oracle as O
-from pargridcpu_b200 import MultilayerGraph, batch_run, synth
+from pargridcpu_b200 import MultilayerGraph, batch_run, native, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -110,3 +110,26 @@ def test_columns_that_leave_in_the_first_scan(monkeypatch):
     for layers in (dense, few, dense):
         ref = O.OracleGraph(layers).coreindex()
         assert np.array_equal(MultilayerGraph.from_pairs(layers).coreindex(), ref)
+
+
+def test_deadline_is_the_whole_run_s(monkeypatch):
+    """A run whose two launches each stay within the deadline and together do
+    not ends with an error, and the next call gets the table."""
+    gen = synth.chung_lu_graph(1_200_000, 4, 8_000_000, 2.1, 0.5, 61)
+    g = MultilayerGraph.from_pairs(gen.layers)
+    monkeypatch.setenv("FC_PEEL_LATE", "100000")
+    ref = g.coreindex()
+    times = []
+    for _ in range(4):
+        g.reset_results()
+        g.coreindex()
+        times.append(g.stats()["peel_ms"])
+    limit = int(0.75 * min(times))
+    assert limit >= 3
+    monkeypatch.setenv("FC_PEEL_DEADLINE_MS", str(limit))
+    g.reset_results()
+    with pytest.raises(native.FcError) as e:
+        g.coreindex()
+    assert e.value.code == 6  # FC_ERR_ITER_LIMIT
+    monkeypatch.delenv("FC_PEEL_DEADLINE_MS")
+    assert np.array_equal(g.coreindex(), ref)
