@@ -516,6 +516,9 @@ __global__ void __launch_bounds__(T, 1) k_late(const __grid_constant__ LateJob j
         }
         if (lead) {
             const uint64_t now = global_ns();
+            c->ph_ns[0] += t_scan - t_last;
+            c->ph_ns[1] += now - t_scan;
+            c->queued += lv_items;
             if (j.trace && k < j.trace_levels) {
                 unsigned long long* r = j.trace + (uint64_t)TRACE_W * k;
                 r[0] = t_scan - t_last;

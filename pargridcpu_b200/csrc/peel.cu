@@ -1165,13 +1165,13 @@ static fc_status run_job(PeelJob& j, const PeelPlan& p, uint32_t threads, cudaSt
         cudaEventDestroy(e1);
     }
     if (st) {
-        st->ms = ms;
+        // times and items of all its launches (a repetition's after the first try's)
+        st->ms += ms;
         st->levels = out.levels + lo[0].levels + lo[1].levels;
-        st->subrounds = out.items;
+        st->subrounds += (uint32_t)(out.items + lo[0].queued + lo[1].queued);
         st->err = out.err.v;
-        st->phase_ms[0] = out.ph_ns[0] * 1e-6;
-        st->phase_ms[1] = out.ph_ns[1] * 1e-6;
-        st->phase_ms[2] = 0;
+        for (int i = 0; i < 2; i++)
+            st->phase_ms[i] += (out.ph_ns[i] + lo[0].ph_ns[i] + lo[1].ph_ns[i]) * 1e-6;
     }
     if (tracing) {
         // one line per level: scan us, expansion us, rounds, queue items, alive nodes

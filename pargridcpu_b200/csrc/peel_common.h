@@ -221,6 +221,8 @@ struct LateCtl {
     uint32_t m, first_level, list, nfill, levels;  // where it starts: nodes, level, list
     uint32_t entries, words;  // row entries and degree words reserved
     uint64_t t_start;   // when the run began
+    uint64_t ph_ns[2];  // time in scans, in expansions
+    uint64_t queued;    // items
 };
 
 // Where the scratch of one run lies.

@@ -133,3 +133,24 @@ def test_deadline_is_the_whole_run_s(monkeypatch):
     assert e.value.code == 6  # FC_ERR_ITER_LIMIT
     monkeypatch.delenv("FC_PEEL_DEADLINE_MS")
     assert np.array_equal(g.coreindex(), ref)
+
+
+@pytest.mark.parametrize("late", [0, 2000, 262144])
+def test_statistics_cover_every_form(late, monkeypatch):
+    """Items and phase times of all the launches of a run, whichever form takes
+    its levels."""
+    monkeypatch.setenv("FC_PEEL_WHOLE", "0")
+    monkeypatch.setenv("FC_PEEL_LATE", str(late))
+    g = MultilayerGraph.from_pairs(graph(20_000, 5, 60_000, 62))
+    ref = O.OracleGraph(graph(20_000, 5, 60_000, 62)).coreindex()
+    assert np.array_equal(g.coreindex(), ref)
+    st = g.stats()
+    # a node is queued at least once for each level that removes it in some
+    # column, unless no survivor is left that its row could name
+    values = np.sort(ref, axis=0)
+    removals = int((np.diff(values, axis=0) != 0).sum()) + g.n
+    assert st["subrounds"] >= removals - int((ref == ref.max()).any(axis=0).sum())
+    assert st["levels"] >= int(ref.max()) + 1
+    scan, expand, _ = st["phase_ms"]
+    assert scan > 0 and expand > 0
+    assert scan + expand <= st["peel_ms"] + 0.1
