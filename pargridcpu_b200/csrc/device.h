@@ -174,6 +174,9 @@ struct PeelGraph {
     // (sizes only) max_level is an upper bound: what is computed for it must do
     // for any smaller one
     bool bound = false;
+    // a row may name a neighbour twice in one layer: degrees and cores past what
+    // the packed fields rely on (65,535 of them, and no more than the nodes)
+    bool repeats = false;
 };
 // scratch bytes one peel launch over `ncols` columns of g needs
 uint64_t peel_ws_bytes(const PeelGraph& g, uint32_t ncols, bool late = false);

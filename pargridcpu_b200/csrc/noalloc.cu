@@ -21,8 +21,10 @@
 // The caller's CSR is checked before the peel reads it: node_ptr must start
 // at 0, never decrease and end at `entries`, and every slot must name one of
 // the n*L degree counters.  Those are the properties the peel's indexing
-// rests on; a violation ends the call with FC_ERR_INVALID.  The check's flag
-// is the last word of the array, outside the peel's scratch.
+// rests on; a violation ends the call with FC_ERR_INVALID.  Rows may repeat a
+// neighbour (the library's own never do), so the check also finds the largest
+// degree: past 16 bits the peel runs on 32-bit degrees.  Both words lie in the
+// array's last 256 bytes, outside the peel's scratch.
 #include <mutex>
 
 #include "device.h"
@@ -30,7 +32,7 @@
 namespace fc {
 
 constexpr size_t FIXED_SCRATCH_BYTES = 64ull << 20;
-// the peel's part; the last 256 bytes hold the input check's flag
+// the peel's part; the last 256 bytes hold the input check's flag and degree
 constexpr size_t PEEL_SCRATCH_BYTES = FIXED_SCRATCH_BYTES - 256;
 
 // The scratch itself.  In host code this name is a host-side stand-in, not a
@@ -59,12 +61,12 @@ static fc_status fixed_scratch(void** out) {
     return FC_OK;
 }
 
-// Bounded input check (grid-stride, no waits): sets *bad when node_ptr does
+// Bounded input check (grid-stride, no waits): sets out[0] when node_ptr does
 // not start at 0, decreases or does not end at `entries`, or a slot is not
-// below nL.
+// below nL; out[1] receives the largest degree.
 __global__ void k_check_csr(const uint32_t* __restrict__ node_ptr, uint32_t n,
                             const uint32_t* __restrict__ adj, uint64_t entries, uint64_t nL,
-                            uint32_t* __restrict__ bad) {
+                            const uint32_t* __restrict__ deg0, uint32_t* __restrict__ out) {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     uint32_t b = 0;
@@ -73,7 +75,11 @@ __global__ void k_check_csr(const uint32_t* __restrict__ node_ptr, uint32_t n,
         if (node_ptr[v + 1] < node_ptr[v]) b = 1;
     for (uint64_t e = t; e < entries; e += stride)
         if (adj[e] >= nL) b = 1;
-    if (__any_sync(0xffffffffu, b) && (threadIdx.x & 31) == 0) atomicOr(bad, 1u);
+    uint32_t m = 0;
+    for (uint64_t i = t; i < nL; i += stride) m = max(m, deg0[i]);
+    m = __reduce_max_sync(0xffffffffu, m);
+    if (__any_sync(0xffffffffu, b) && (threadIdx.x & 31) == 0) atomicOr(out, 1u);
+    if ((threadIdx.x & 31) == 0 && m) atomicMax(out + 1, m);
 }
 
 }  // namespace fc
@@ -92,26 +98,33 @@ extern "C" fc_status fc_coreindex_fixed_scratch(uint32_t n, uint32_t n_layers, u
     // whose single column does not fit is rejected before any device work
     uint32_t cols = n_layers;
     // core <= largest degree <= n - 1 bounds the level count
-    const PeelGraph g{n, n_layers, entries, node_ptr, adj, deg0, n + 1};
+    PeelGraph g{n, n_layers, entries, node_ptr, adj, deg0, n + 1};
     // (with the form for a peel's last levels when all columns fit with it)
-    const bool late = peel_ws_bytes(g, cols, true) <= PEEL_SCRATCH_BYTES;
+    bool late = peel_ws_bytes(g, cols, true) <= PEEL_SCRATCH_BYTES;
     while (!late && cols > 0 && peel_ws_bytes(g, cols) > PEEL_SCRATCH_BYTES) cols--;
     if (cols == 0) return FC_ERR_TOO_LARGE;
     void* ws = nullptr;
     FC_TRY(fixed_scratch(&ws));
     cudaStream_t s = (cudaStream_t)stream;
     {
-        uint32_t* bad = (uint32_t*)((char*)ws + PEEL_SCRATCH_BYTES);
-        FC_CUDA_TRY(cudaMemsetAsync(bad, 0, 4, s));
+        uint32_t* out = (uint32_t*)((char*)ws + PEEL_SCRATCH_BYTES);
+        FC_CUDA_TRY(cudaMemsetAsync(out, 0, 8, s));
         int dev = 0, sms = 0;
         FC_CUDA_TRY(cudaGetDevice(&dev));
         FC_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        k_check_csr<<<sms * 4, 256, 0, s>>>(node_ptr, n, adj, entries, (uint64_t)n * n_layers, bad);
+        k_check_csr<<<sms * 4, 256, 0, s>>>(node_ptr, n, adj, entries, (uint64_t)n * n_layers, deg0,
+                                           out);
         count_launch();
         FC_CUDA_TRY(cudaGetLastError());
-        uint32_t flag = 0;
-        FC_TRY(to_host(&flag, bad, 4, s));
-        if (flag) return FC_ERR_INVALID;
+        uint32_t found[2] = {0, 0};
+        FC_TRY(to_host(found, out, 8, s));
+        if (found[0]) return FC_ERR_INVALID;
+        g.repeats = found[1] > 0xFFFFu;
+    }
+    if (g.repeats) {  // (a column alone, which fits, never has more than 32 bits a degree)
+        late = false;
+        cols = n_layers;
+        while (cols > 1 && peel_ws_bytes(g, cols) > PEEL_SCRATCH_BYTES) cols--;
     }
     for (uint32_t c0 = 0; c0 < n_layers; c0 += cols) {
         const uint32_t nc = n_layers - c0 < cols ? n_layers - c0 : cols;

@@ -854,11 +854,12 @@ uint32_t peel_kind(const PeelGraph& g) {
 // kept apart from those of the steps around it.  Unpacked (one column per
 // segment, 32-bit degrees, one queue): when every spec is a single column and
 // no late form follows, where packing would only waste the other three fields,
-// and when a count of layers does not fit a field.
+// when a count of layers does not fit a field, and when a degree may pass it
+// without as many nodes.
 static bool packs(const PeelSegSpec* specs, size_t count, bool late) {
     bool several = late;
     for (size_t i = 0; i < count; i++) {
-        if (specs[i].g.L > MAX_PACKED_LAYERS) return false;
+        if (specs[i].g.L > MAX_PACKED_LAYERS || specs[i].g.repeats) return false;
         several |= specs[i].ncols > 1;
     }
     return several;

@@ -159,3 +159,47 @@ def test_fixed_scratch_rejects_a_malformed_csr():
     assert _call(n, L, e, _dev(node_ptr), _dev(slots), _dev(deg0), out) == FC_OK
     torch.cuda.synchronize()
     assert np.array_equal(out.cpu().numpy().view(np.uint32), ref)
+
+
+def _multigraph_cores(A):
+    """core_lambda by definition from the layers' matrices of edge counts."""
+    L, n, _ = A.shape
+    out = np.zeros((L, n), np.uint32)
+    for lam in range(1, L + 1):
+        alive, k = np.ones(n, bool), 0
+        while alive.any():
+            while True:
+                deg = A[:, :, alive].sum(axis=2)
+                gone = alive & ((deg >= k + 1).sum(axis=0) < lam)
+                if not gone.any():
+                    break
+                out[lam - 1, gone] = k
+                alive &= ~gone
+            k += 1
+    return out
+
+
+@pytest.mark.parametrize("times", [200, 218, 219, 290])
+def test_fixed_scratch_degrees_past_sixteen_bits_with_few_nodes(times):
+    """The preconditions allow rows that repeat a neighbour: a hub of 300
+    leaves with `times` edges to each has up to 87,000 entries in one layer."""
+    import torch
+    n, L = 301, 2
+    rng = np.random.default_rng(times)
+    A = np.zeros((L, n, n), np.int64)
+    A[0, 0, 1:] = A[0, 1:, 0] = times
+    ring = np.arange(1, n)
+    for u, v in zip(ring, np.roll(ring, 1)):
+        A[1, u, v] = A[1, v, u] = int(rng.integers(1, 40))
+    deg0 = np.ascontiguousarray(A.sum(axis=2).T.astype(np.uint32)).reshape(-1)
+    slots, node_ptr = [], [0]
+    for v in range(n):
+        for l in range(L):
+            slots.append(np.repeat(np.arange(n) * L + l, A[l, v]))
+        node_ptr.append(sum(len(s) for s in slots[-L:]) + node_ptr[-1])
+    slots = np.concatenate(slots).astype(np.uint32)
+    out = torch.empty((L, n), dtype=torch.int32, device="cuda")
+    rc = _call(n, L, len(slots), _dev(np.array(node_ptr, np.uint32)), _dev(slots), _dev(deg0), out)
+    torch.cuda.synchronize()
+    assert rc == FC_OK, native.STATUS.get(rc, rc)
+    assert np.array_equal(out.cpu().numpy().view(np.uint32), _multigraph_cores(A))
