@@ -53,3 +53,13 @@ def test_a_column_whose_bins_fit_no_block():
     rng = np.random.default_rng(9)
     some = [np.unique(rng.integers(0, 640, (40, 2)), axis=0) for _ in range(199)]
     check([clique(np.arange(640))] + [p[p[:, 0] != p[:, 1]].astype(np.uint32) for p in some])
+
+
+def test_more_column_groups_than_one_launch_holds():
+    # 420 columns with cores of 44 to 78: 118 groups, 64 a launch
+    layers = synth.erdos_renyi_graph(120, 420, 0.55, 0.55, 77).layers
+    g, og = MultilayerGraph.from_pairs(layers), O.OracleGraph(layers)
+    ref = og.densest(og.coreindex(), 1.0)
+    rec, dens = g.cells(1.0)
+    assert np.array_equal(rec, ref["cells"])
+    assert np.array_equal(dens.view(np.uint64), ref["cell_density"].view(np.uint64))

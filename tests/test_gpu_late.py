@@ -154,3 +154,16 @@ def test_statistics_cover_every_form(late, monkeypatch):
     scan, expand, _ = st["phase_ms"]
     assert scan > 0 and expand > 0
     assert scan + expand <= st["peel_ms"] + 0.1
+
+
+@pytest.mark.parametrize("late", [None, 0, 40_000])
+def test_batch_with_a_graph_of_degrees_past_sixteen_bits(late, monkeypatch):
+    if late is not None:
+        monkeypatch.setenv("FC_PEEL_LATE", str(late))
+    leaves = 70_001
+    star = np.stack([np.zeros(leaves, np.int64), 1 + np.arange(leaves)], 1).astype(np.uint32)
+    inputs = [graph(900, 6, 3000, 55), [star] + graph(leaves, 2, 2 * leaves, 56),
+              graph(1500, 1, 5000, 57)]
+    tables, _, _ = batch_run([MultilayerGraph.from_pairs(x) for x in inputs])
+    for layers, table in zip(inputs, tables):
+        assert np.array_equal(table, O.OracleGraph(layers).coreindex())

@@ -203,3 +203,20 @@ def test_fixed_scratch_degrees_past_sixteen_bits_with_few_nodes(times):
     torch.cuda.synchronize()
     assert rc == FC_OK, native.STATUS.get(rc, rc)
     assert np.array_equal(out.cpu().numpy().view(np.uint32), _multigraph_cores(A))
+
+
+def test_fixed_scratch_in_column_groups():
+    """More columns than the array holds at once: they run in groups, the last
+    one shorter."""
+    import torch
+    gen = synth.chung_lu_graph(300_000, 11, 120_000, 2.2, 0.4, 9095)
+    g = MultilayerGraph.from_pairs(gen.layers)
+    node_ptr, slots, deg0 = node_major(g)
+    d_ptr, d_adj, d_deg0 = _dev(node_ptr), _dev(slots), _dev(deg0)
+    out = torch.empty((g.L, g.n), dtype=torch.int32, device="cuda")
+    before = native.lib().fc_launch_count()
+    assert _call(g.n, g.L, len(slots), d_ptr, d_adj, d_deg0, out) == FC_OK
+    # the check and at least two peels
+    assert native.lib().fc_launch_count() - before >= 3
+    torch.cuda.synchronize()
+    assert np.array_equal(out.cpu().numpy().view(np.uint32), g.coreindex())
