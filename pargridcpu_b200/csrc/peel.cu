@@ -782,21 +782,6 @@ static uint32_t env_u32(const char* name, uint32_t dflt) {
     return s && *s ? (uint32_t)strtoul(s, nullptr, 10) : dflt;
 }
 
-uint32_t peel_columns_per_group(const DeviceGraph* d) {
-    // a column needs 2 bytes per (node, layer) and a few words per node; keep
-    // the group's working set within a budget (FC_PEEL_GROUP_MB, default 4 GiB)
-    const uint64_t per_col = ((uint64_t)d->n * d->L + 4ull * d->n) * 2 + d->entries / 64;
-    const uint64_t budget = (uint64_t)env_u32("FC_PEEL_GROUP_MB", 4096) << 20;
-    uint64_t cols = per_col ? budget / per_col : d->L;
-    uint32_t want = env_u32("FC_PEEL_GROUP_COLS", 0);
-    if (want) cols = want;
-    if (cols < 1) cols = 1;
-    if (cols > d->L) cols = d->L;
-    // the (column, node) index must stay below 2^32
-    while (cols > 1 && (uint64_t)cols * d->n >= (1ull << 32)) cols--;
-    return (uint32_t)cols;
-}
-
 template <int T, bool MULTI, bool PACK, int BPS = 1024 / T>
 static fc_status launch_t(PeelJob& j, cudaStream_t s) {
     int dev = 0, sms = 0, occ = 0;
@@ -1012,6 +997,26 @@ static uint64_t run_bytes(const PeelSegSpec* specs, size_t count, bool late) {
         bytes = std::max(bytes, q.total);
     }
     return bytes;
+}
+
+// As many columns as keep the peel's scratch within a budget
+// (FC_PEEL_GROUP_MB, default 4 GiB); the late form's comes on top.
+uint32_t peel_columns_per_group(const DeviceGraph* d) {
+    const PeelGraph g{d->n, d->L, d->entries, nullptr, nullptr, nullptr, d->max_deg + 1};
+    const uint64_t budget = (uint64_t)env_u32("FC_PEEL_GROUP_MB", 4096) << 20;
+    uint32_t cols = std::min(env_u32("FC_PEEL_GROUP_COLS", 0), d->L);
+    if (!cols) {
+        uint32_t fit = 0, no = d->L + 1;  // cols in [fit, no)
+        for (cols = d->L; no - fit > 1; cols = fit + (no - fit) / 2) {
+            if (cols <= 1 || peel_ws_bytes(g, cols) <= budget) fit = cols;
+            else no = cols;
+        }
+        cols = fit;
+    }
+    if (cols < 1) cols = 1;
+    // the (column, node) index must stay below 2^32
+    while (cols > 1 && (uint64_t)cols * d->n >= (1ull << 32)) cols--;
+    return cols;
 }
 
 uint64_t peel_ws_bytes(const PeelGraph& g, uint32_t ncols, bool late) {

@@ -9,6 +9,11 @@
 // lets the graphs join a server's batch one after another and prints what its
 // admission charges for the batch's scratch, whether it runs without the late
 // form, the most scratch that its launches take, and the graphs that joined.
+//
+//   plan_check group BUDGET n,L,entries,largest_degree
+//
+// prints the columns that a graph's peel takes at once (FC_PEEL_GROUP_MB in the
+// environment), their scratch and that of one column more.
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
@@ -41,6 +46,18 @@ int main(int argc, char** argv) {
     }
     if (!strcmp(argv[1], "scratch")) {
         printf("%llu\n", (unsigned long long)peel_batch_ws_bytes(specs, atoi(argv[2]) != 0));
+        return 0;
+    }
+    if (!strcmp(argv[1], "group")) {
+        DeviceGraph d;
+        const PeelGraph& g = specs[0].g;
+        d.n = g.n;
+        d.L = g.L;
+        d.entries = g.entries;
+        d.max_deg = g.max_level - 1;
+        const uint32_t cols = peel_columns_per_group(&d);
+        printf("%u %llu %llu\n", cols, (unsigned long long)peel_ws_bytes(g, cols),
+               (unsigned long long)peel_ws_bytes(g, std::min(cols + 1, g.L)));
         return 0;
     }
     const uint64_t budget = strtoull(argv[2], nullptr, 10);

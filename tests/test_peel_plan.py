@@ -95,3 +95,19 @@ def test_a_request_that_does_not_fit_does_not_change_the_batch(plan):
     assert (lean, joined) == (0, 2) and charged == taken
     charged, lean, taken, joined = plan("admit", budget, [large, small])
     assert (lean, joined) == (1, 1) and charged >= taken
+
+
+@pytest.mark.parametrize("graph", [(100_000_000, 4, 400_000_000, 500),
+                                   (2_600_000, 24, 96_000_000, 5000),
+                                   (9_000_000, 60, 900_000_000, 5000),
+                                   (60_000, 33_000, 200_000_000, 500),
+                                   (2_400_000, 4, 68_000_000, 900_000),
+                                   (3000, 1, 20_000, 50)])
+@pytest.mark.parametrize("mb", [64, 4096])
+def test_column_groups_keep_their_budget(plan, graph, mb):
+    """A group is one column, or its scratch is within the budget and as many
+    columns as fit it."""
+    cols, bytes_, more = plan("group", 0, [graph], FC_PEEL_GROUP_MB=mb)
+    assert 1 <= cols <= graph[1]
+    assert cols == 1 or bytes_ <= mb << 20
+    assert cols == graph[1] or more > mb << 20 or (cols + 1) * graph[0] >= 1 << 32
