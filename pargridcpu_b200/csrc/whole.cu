@@ -233,7 +233,6 @@ __global__ void __launch_bounds__(WH_THREADS) k_whole(
 // another may still reach its shared memory.
 // Rows longer than CL_SPLIT entries are expanded by every block, a slice each.
 constexpr uint32_t CL_SPLIT = 2048;
-constexpr uint32_t CL_MAX = 16;
 // The count half of a node that is not kept in the current level: decrements
 // of a removed node's count (at most L, one per layer degree passing k + 1)
 // leave it far above any lmd, and never borrow (L is at most 96 here: a
