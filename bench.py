@@ -377,7 +377,8 @@ def run_ours(args, world, rank, local):
         step()
     probe = None
     if not args.no_probe and rank == 0:
-        probe = atomic_probe(4 * n * L * min(L, max(my_cols, 1)))
+        # four columns' degrees share an 8-byte word
+        probe = atomic_probe(8 * n * L * ((min(L, max(my_cols, 1)) + 3) // 4))
     clocks = Clocks(local)
     barrier()
     clocks.start()
@@ -507,7 +508,8 @@ def run_ours(args, world, rank, local):
     if rank != 0:
         return
     # roofline of the dominant stage (the peel: k_peel and the late form that
-    # finishes the columns, or takes every level): algorithmic bytes
+    # finishes the columns, or takes every level; or a block or cluster per
+    # column, which counts no items): algorithmic bytes
     # per launch (bytes_per_column per lambda column) over the mean CUDA-event
     # time of a launch
     cols = min(stats["columns_per_launch"] or L, max(my_cols, 1))
@@ -520,7 +522,8 @@ def run_ours(args, world, rank, local):
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak, "traffic": traffic,
             "kernel": "k_peel + late form (k_lt_rows, k_lt_degrees, k_lt_fill, k_lt_fill_long, "
-                      "k_late)", "peak_kind": peak_kind,
+                      "k_late)" if stats["subrounds"] else "k_whole or k_whole_cl",
+            "peak_kind": peak_kind,
             "bytes_per_launch": bytes_per_launch, "launch_ms": launch_ms,
             # atomics are reported beside the bytes, not folded in
             "l2_atomic_sectors_per_launch": atom_sectors,
@@ -741,7 +744,7 @@ def run_batch(args, world, rank, local):
                                        else "single process")},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": None,
-                         "kernel": "k_peel<1,T,true> (batched, all graphs' columns)",
+                         "kernel": "k_peel + late form (batched, all graphs' columns)",
                          "peak_kind": peak_kind, "bytes_per_launch": bytes_launch,
                          "launch_ms": peel_ms},
             "e2e": e2e, "gpu_launches": launches, "clocks": clk,

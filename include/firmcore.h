@@ -238,10 +238,9 @@ fc_status fc_mlcd_query(const uint32_t* cores, uint32_t n, uint32_t P, const uin
                         uint64_t cap, void* stream);
 
 /* ---- batch ---------------------------------------------------------------
- * Many graphs at once: all (graph, lambda) columns in one persistent kernel
- * launch whose warps pull work items from device queues (captured in a CUDA
- * graph when use_cuda_graph is set), then the densest search for `beta` on
- * every graph.  tables[i] (host, may be NULL) receives graph i's L*n table,
+ * Many graphs at once: all (graph, lambda) columns share one level loop on the
+ * whole device (its launches captured in a CUDA graph when use_cuda_graph is
+ * set), then the densest search for `beta` on every graph.  tables[i] (host, may be NULL) receives graph i's L*n table,
  * res[i] (may be NULL) its densest result.  The equivalent of running the
  * reference once per graph; every result is identical to fc_coreindex +
  * fc_densest on the graph alone.  With `plain` set it runs the baseline
@@ -358,7 +357,7 @@ fc_status fc_server_destroy(fc_server* s);
  * violation returns FC_ERR_INVALID with nothing else done); the others
  * decide only the values of the table.
  * A graph whose one column needs more than the array's scratch (about
- * 4*n*L + 36*n + entries/16 bytes) is rejected with FC_ERR_TOO_LARGE before
+ * 4*n*L + 28*n + entries/32 bytes) is rejected with FC_ERR_TOO_LARGE before
  * any device work.  A call cannot be captured in a CUDA graph: it reads the
  * run's status back on the host (a copy and a stream synchronization) before
  * it returns.  All calls share the one array per device, so
