@@ -220,3 +220,37 @@ def test_fixed_scratch_in_column_groups():
     assert native.lib().fc_launch_count() - before >= 3
     torch.cuda.synchronize()
     assert np.array_equal(out.cpu().numpy().view(np.uint32), g.coreindex())
+
+
+@pytest.mark.parametrize("twice", [0, 1, 3000])
+def test_fixed_scratch_hub_with_and_without_repeats(twice):
+    """One layer: a hub of 70,000 leaves, the last `twice` of them joined to it
+    by two edges, so that a leaf's core is its edges' number."""
+    import torch
+    n = 70_001
+    times = np.ones(n - 1, np.int64)
+    times[n - 1 - twice:] = 2
+    deg0 = np.concatenate([[times.sum()], times]).astype(np.uint32)
+    node_ptr = np.concatenate([[0], np.cumsum(deg0.astype(np.int64))]).astype(np.uint32)
+    slots = np.concatenate([np.repeat(np.arange(1, n), times), np.zeros(times.sum(), np.int64)])
+    out = torch.empty((1, n), dtype=torch.int32, device="cuda")
+    rc = _call(n, 1, len(slots), _dev(node_ptr), _dev(slots.astype(np.uint32)), _dev(deg0), out)
+    torch.cuda.synchronize()
+    assert rc == FC_OK, native.STATUS.get(rc, rc)
+    want = np.concatenate([[times.max()], times]).astype(np.uint32)
+    assert np.array_equal(out.cpu().numpy().view(np.uint32)[0], want)
+
+
+def test_fixed_scratch_hub_graph():
+    import torch
+    star = np.stack([np.full(70_000, 3), 4 + np.arange(70_000)], 1).astype(np.uint32)
+    layers = list(synth.chung_lu_graph(90_000, 4, 100_000, 2.3, 0.4, 9096).layers)
+    layers[1] = np.concatenate([layers[1], star])
+    layers[2] = np.concatenate([layers[2], star])
+    g = MultilayerGraph.from_pairs(layers)
+    node_ptr, slots, deg0 = node_major(g)
+    assert (deg0 > 65_535).sum() == 2
+    out = torch.empty((g.L, g.n), dtype=torch.int32, device="cuda")
+    assert _call(g.n, g.L, len(slots), _dev(node_ptr), _dev(slots), _dev(deg0), out) == FC_OK
+    torch.cuda.synchronize()
+    assert np.array_equal(out.cpu().numpy().view(np.uint32), g.coreindex())
